@@ -121,12 +121,12 @@ int kyb_gemm_kq_ag(int fmt, const void* t16, int64_t n, int64_t k, const void* a
 int kyb_gemm_nvfp4_ag(const void* a_codes, const void* sfa, const void* b_codes, const void* sfb, int64_t m, int64_t n, int64_t k, float gscale, int out_dtype,
                       const kyb_peer_out* out, int64_t ldd, int64_t col0, void* stream);
 
-/* ---- prefill GEMM with the dequantisation fused into the tensor-core operand producer: weights are read as T16 tiles and decoded into shared memory, the fp16
+/* ---- prefill GEMM with the dequantisation fused into the tensor-core operand producer: weights are read as T16 tiles and decoded into tensor memory, the fp16
  * matrix never exists in HBM. d fp16 [m, n] = sat(gscale * a fp16 [m, k] x W^T). Same call sites as the two entries above
  * (kyojin_mlx/foreign_linear.py:710 / :737 dense, kyojin_mlx/foreign_kqgmm.py:225-239 `gmm` grouped). Weights are rounded to fp16 at the reference's own rounding
  * points for its few-row tensor kernels (block scale and min to fp16, one fp16 fma per weight: kyojin_mlx/foreign_metal.py:1357-1358, :1382-1383); NVFP4 weights
- * are exact in fp16. msub = 0: chosen by the library (CTA pairs, tcgen05 cta_group::2, for more than 128 rows and one destination); 1 or 2: the one-CTA
- * kernel with that many 128-row blocks of a per work item (same bits either way). The grouped form needs n % 256 == 0 and tb / off from
+ * are exact in fp16. msub = 0: chosen by the library (CTA pairs, tcgen05 cta_group::2, unless the one-CTA form fills the SMs better); 1 or 2: the one-CTA
+ * form with up to that many 128-row blocks of a per work item (same bits either way). The grouped form needs n % 256 == 0 and tb / off from
  * kyb_moe_plan with the same mt (128 or 256 rows of one expert per work item). */
 int kyb_gemm_kq(int fmt, const void* t16, int64_t n, int64_t k, const void* a, int64_t lda, int64_t m, float gscale, void* d, int64_t ldd, int msub, void* stream);
 /* split-k form of kyb_gemm_kq for products with fewer 256 x 256 output tiles than SMs (the reference has no counterpart: its fallback for these row counts is
@@ -140,8 +140,8 @@ int kyb_gemm_kq_splitk(int fmt, const void* t16, int64_t n, int64_t k, const voi
                        void* workspace, size_t workspace_bytes, void* stream);
 int kyb_gemm_kq_grouped(int fmt, const void* t16, int64_t n, int64_t k, int experts, const void* a, int64_t lda, int64_t s, const void* tb, const void* off,
                         const void* row_map, const void* gs, void* d, int64_t ldd, int mt, void* stream);
-/* gate and up of a routed SwiGLU layer as ONE grouped product with the gated activation in its epilogue: an item's 256 weight rows are 128 rows of the gate stack
- * and the same 128 rows of the up stack; h fp16 [s, n] (sorted order) = silu(a) * b of the two products rounded to fp16 (what two kyb_gemm_kq_grouped calls would
+/* gate and up of a routed SwiGLU layer as ONE grouped product with the gated activation in its epilogue: the weight rows of an item are half rows of the gate stack,
+ * half the same rows of the up stack; h fp16 [s, n] (sorted order) = silu(a) * b of the two products rounded to fp16 (what two kyb_gemm_kq_grouped calls would
  * store), optional clamp `limit` as kyb_silu_mul. Replaces gmm, gmm, silu_perm of kyojin_mlx/foreign_kqgmm.py:293-314 `mlp`. n % 128 == 0, ldh % 8 == 0. */
 int kyb_gemm_kq_grouped_glu(int fmt, const void* t16_gate, const void* t16_up, int64_t n, int64_t k, int experts, const void* a, int64_t lda, int64_t s, const void* tb,
                             const void* off, const void* gs_gate, const void* gs_up, float limit, void* h, int64_t ldh, int mt, void* stream);

@@ -2,18 +2,32 @@
 // (every format of the library) and never written to HBM as fp16. Replaces the two-step large-row path of kyojin_mlx/foreign_linear.py:710 / :737
 // (`x2 @ self.dequant().T`) and, in grouped form, the sorted grouped product of kyojin_mlx/foreign_kqgmm.py:225-239 (`gmm`).
 //
+// The weights are the M-side operand and live in tensor memory: the decoders' registers are already the 16 x 256-bit fragments that `tcgen05.st.16x256b` stores (a
+// T16 row tile is 16 rows; lane (g, t) holds four consecutive inputs of rows g and g + 8 of every 16-input slice), so one store instruction per 16 rows x 64 inputs
+// replaces eight swizzled shared-memory stores and their selects, and neither the decoded weights nor the MMA's reads of them touch shared memory. The activations
+// are the N-side operand (TMA, 128-byte swizzle), so an item costs MMA time in proportion to its rows (N = rows rounded up to 16; 32 by pairs) instead of whole
+// 128-row blocks, and the accumulator holds D transposed (lanes = outputs, columns = activation rows).
+//
 // One persistent CTA per SM, 22 warps:
-//   warp 0      TMA: activation tiles (128 rows x 64 inputs, 128-byte swizzle) into the stage ring
-//   warp 1      tcgen05.mma issuer (UMMA 128 x 256 x 16, kind::f16, fp32 accumulators in tensor memory), stages handed back by tcgen05.commit
-//   warps 2-5   epilogue: tcgen05.ld, output scale, saturating fp16 stores
-//   warps 6-21  decoders: warp w owns the 16-row T16 row tile w of the CTA's 256 weight rows. It keeps one T16 tile (256 inputs) in registers (the next one
-//               is already in flight), and for each 64-input quarter unpacks the codes with LOP3 / PRMT into fp16 pairs, applies the block scales with
-//               half2 arithmetic (scale and min rounded to fp16, then one fma per pair: the rounding points of the reference's few-row kernels,
-//               kyojin_mlx/foreign_metal.py:1357-1358, :1382-1383) and writes the pairs into the stage's B tile in the swizzled K-major layout the UMMA
-//               descriptor expects, followed by a proxy fence and one mbarrier arrival per warp.
-// A work item is a 256-row block of W times one or two 128-row blocks of A (msub): with two, a decoded weight serves 256 activation rows, which halves the
-// decode work per flop; with one, the two tensor-memory accumulators alternate and the epilogue overlaps the next item's MMAs (grouped form: an expert's
-// segment is cut into 128-row tiles). Every mbarrier wait is bounded; a wait that gives up sets the device status word and the CTA drains.
+//   warp 0      TMA: activation boxes (64 rows x 64 inputs) into a ring of shared-memory stages
+//   warp 1      tcgen05.mma issuer (M = 128 output rows, A from tensor memory, two accumulator slots of 128 columns), tcgen05.commit hands stages back
+//   warps 2-5   epilogue: tcgen05.ld 16x256b, output scale, stmatrix.trans turns the fragments around into [activation row][output] staging tiles, which leave as
+//               tiled bulk stores or as coalesced row pieces
+//   warps 6-21  decoders: warp (q = warp % 4, j) owns row tile 2 q + (j & 1) of the CTA's 128 output rows (the tensor-memory lanes a warp may touch are those of its
+//               quarter q) and every second T16 tile of it (parity j >> 1). It keeps one T16 tile in registers, each unit refilled from its next tile right after its
+//               use (across items too), unpacks a 64-input quarter with LOP3 / PRMT into fp16 pairs, applies the block scales with half2 arithmetic (scale and
+//               min rounded to fp16, then one fma per pair: the rounding points of the reference's few-row kernels, kyojin_mlx/foreign_metal.py:1357-1358,
+//               :1382-1383) and stores it into one of eight tensor-memory stages (32 columns each).
+// PAIR (tcgen05 cta_group::2): two CTAs of neighbouring SMs compute 256 outputs; each decodes its own 128 rows into its own tensor memory and loads half of the
+// activation rows, one MMA of the leader (cluster rank 0) drives both tensor cores. full barriers, acc_empty in the leader; empty and acc_full in each CTA
+// (commit to the pair). Remote arrivals use the plain (CTA-scope release) form: what they publish sits in the arriving CTA's own tensor memory.
+// Every mbarrier wait is bounded; a wait that gives up sets the device status word and the CTA drains.
+//
+// What bounds it: wide items (N = 256) the tensor core and, in a long run of them, the power limit; narrow ones the chain of the decoders and of the two issuing warps
+// (about 350 clocks per 64 inputs of 128 outputs). Measured against the form with the decoded weights in shared memory (same box, back-to-back launches):
+// Q4_K 13824 x 5120, 96 rows 50.6 -> 24.8 us; 18944 x 7168, 32 / 128 rows 84 / 85 -> 37 / 43 us; Q6_K 5120 x 27648, 300 rows 146 -> 114 us; Q3_K 3072 x 12288,
+// 2048 rows 169 -> 141 us; Q4_K 16384 x 7168, 4001 rows 826 -> 782 us (power-limited; 664 us in a short burst); 256 experts of 2048 x 7168, 4096 tokens x 8: gate
+// and up 2684 -> 1945 us, down 1450 -> 1264 us. The sums are the same bits: the MMA adds the same products in the same order with its operands exchanged.
 #include <algorithm>
 #include <cstring>
 #include <mutex>
@@ -23,11 +37,12 @@
 
 namespace kyb {
 
-constexpr int KQ_BN = 256, KQ_BK = 64, KQ_DW = 16, KQ_THREADS = (6 + KQ_DW) * 32;
-constexpr uint32_t KQ_A_SUB = 128 * KQ_BK * 2, KQ_B_BYTES = KQ_BN * KQ_BK * 2;
-constexpr int KQ_TORD = 2048;                          // grouped form: tile order table in shared memory (u16 entries)
+constexpr int KQ_BN = 128, KQ_BK = 128, KQ_DW = 16, KQ_THREADS = (6 + KQ_DW) * 32;  // output rows per CTA, inputs per stage
+constexpr int KQ_SA = 4;                                // weight stages in tensor memory: two T16 tiles, one per decoder parity
+constexpr uint32_t KQ_COL_A = 256;                      // tensor memory: accumulator slots [0, 128) and [128, 256), weight stage s at 256 + 64 s
+constexpr int KQ_TORD = 2048;                           // grouped form: tile order table in shared memory (u16 entries)
 constexpr uint32_t KQ_SCR = 1280;                       // per decoder warp: block scales of one T16 tile as half2 pairs
-constexpr uint32_t KQ_STG = KYB_STG_BYTES;              // per epilogue warp: 32 rows x 32 fp16 columns staged for a tiled bulk store
+constexpr uint32_t KQ_STG = 8192;                       // epilogue staging tile: 32 activation rows x 128 outputs as two 128-byte-swizzled halves; two of them
 using KqOutMaps = KybOutMaps;                           // dense form: the [m, col0 + n] fp16 output matrix of every receiving rank
 
 struct KqParams {
@@ -36,25 +51,29 @@ struct KqParams {
     int nout;
     int64_t ldd;
     int m, n, k, nb;            // rows of A, rows of one W matrix, inputs, 256-input blocks
-    int rt_total;               // 16-row tiles in the whole T16 buffer (row tiles past it are clamped; their columns are never stored)
+    int rt_total;               // 16-row tiles in the whole T16 buffer (row tiles past it are clamped; their outputs are never stored)
     float gscale;
     unsigned int* status;
-    const uint32_t* tb;         // grouped form: first (128 msub)-row tile of every expert (E + 1 entries), else null
+    const uint32_t* tb;         // grouped form: first mt-row tile of every expert (E + 1 entries), else null
     const uint32_t* off;        // grouped form: first sorted row of every expert (E + 1 entries)
     const uint32_t* row_map;    // optional: output row of every sorted row
     const float* gs;            // optional: per-expert output scale
     int experts;
     int tiles_m, tiles_n;
-    int msub, stages;
-    int tma_out, col0;          // dense form: the epilogue stores through the tensor maps (bulk tiled stores), at column col0 + n0
-    int wide;                   // ... in 32 x 64 boxes (4 KB of staging per epilogue warp) instead of 32 x 32: used when the tiles also go to other GPUs
-    // gated pair (grouped form): an item's 256 weight rows are 128 rows of the gate stack (t16) and the same 128 rows of the up stack (t16b); the epilogue writes
-    // fp16(silu(a) * b) of the two fp16-rounded products, 128 output columns per item (kyojin_mlx/foreign_kqgmm.py:293-314 `mlp`: gmm, gmm, silu_perm in one launch)
+    int mt;                     // activation rows per item (multiple of 32, at most 256)
+    int bstages;                // shared-memory ring: 4 stages, or 2 of twice the size, of `bstage_bytes` (two halves of 64 inputs)
+    uint32_t bstage_bytes;
+    uint32_t box_rows;          // activation rows per TMA box (64 inputs wide)
+    int tma_out, col0;          // dense form: the epilogue stores through the tensor maps (tiled bulk stores of 32 rows x 64 outputs), at column col0 + n0
+    int vec_out;                // row stores: 16-byte pieces are aligned in every destination
     // split-k (dense form, one destination): the k-blocks are cut into ksplit equal ranges, an item is (tile, range) and writes its fp32 accumulator to
     // part [range][m][ldp] instead of d; gemm_kq_reduce_kernel adds the ranges in k order, scales, saturates and stores d
-    int ksplit, mpad;           // mpad: rows of a range in part (m rounded up to whole items)
+    int ksplit, mpad;           // mpad: rows of a range in part
     float* part;
     int64_t ldp;
+    // gated pair (grouped form): an item's 128 weight rows are 64 rows of the gate stack (t16) and the same 64 rows of the up stack (t16b), 16-row tiles alternating,
+    // so that one epilogue thread holds both products of an output; it writes fp16(silu(a) * b) of the two fp16-rounded products
+    // (kyojin_mlx/foreign_kqgmm.py:293-314 `mlp`: gmm, gmm, silu_perm in one launch)
     const uint8_t* t16b;
     const float* gsb;           // per-expert output scale of the up stack (or null)
     int glu;
@@ -62,15 +81,18 @@ struct KqParams {
 };
 
 struct KqItem {
-    int m0, m_end, n0, b_rt0, nsub;
+    int m0, m_end, n0;          // first activation row, end of the rows that may be stored, first output of this CTA
+    int rt0;                    // T16 row tile of output n0
+    int nn;                     // MMA width: the item's rows rounded up
     int tb0, ntb, sp;           // first 256-input block, number of blocks and index of the item's k-range (the whole of k without split-k)
     float gscale, gscale_b;
     bool valid;
 };
 
-__device__ __forceinline__ KqItem kq_item(const KqParams& p, int t, const uint16_t* tord = nullptr) {
+template <bool PAIR>
+__device__ __forceinline__ KqItem kq_item(const KqParams& p, int t, uint32_t rank, const uint16_t* tord = nullptr) {
     KqItem it;
-    it.valid = true, it.gscale = p.gscale, it.gscale_b = p.gscale, it.m_end = p.m;
+    it.valid = true, it.gscale = p.gscale, it.gscale_b = p.gscale;
     it.tb0 = 0, it.ntb = p.nb, it.sp = 0;
     if (!p.tb) {
         if (p.ksplit > 1) {                                                             // tiles fastest, k-ranges slowest
@@ -79,27 +101,28 @@ __device__ __forceinline__ KqItem kq_item(const KqParams& p, int t, const uint16
             it.ntb = p.nb / p.ksplit, it.tb0 = it.sp * it.ntb;
         }
         const int tn = t / p.tiles_m, tm = t - tn * p.tiles_m;                         // m fastest: CTAs running together share the weight rows
-        it.n0 = tn * KQ_BN, it.m0 = tm * 128 * p.msub, it.b_rt0 = it.n0 >> 4;
-        it.nsub = min(p.msub, (p.m - it.m0 + 127) >> 7);
+        it.n0 = (PAIR ? 2 * tn + (int)rank : tn) * KQ_BN;
+        it.m0 = tm * p.mt, it.m_end = min(p.m, it.m0 + p.mt), it.rt0 = it.n0 >> 4;
+        it.nn = PAIR ? (it.m_end - it.m0 + 31) & ~31 : (it.m_end - it.m0 + 15) & ~15;
         return it;
     }
     int tm = t / p.tiles_n;
     const int tn = t - tm * p.tiles_n;                                                   // n fastest: CTAs running together share the activation rows
-    it.n0 = tn * (p.glu ? KQ_BN / 2 : KQ_BN);
+    it.n0 = (PAIR ? 2 * tn + (int)rank : tn) * (p.glu ? KQ_BN / 2 : KQ_BN);
     if ((uint32_t)tm >= p.tb[p.experts]) {
         it.valid = false;
         return it;
     }
-    if (tord) tm = (int)tord[tm];                                                        // two-block tiles first (see the kernel's prologue)
+    if (tord) tm = (int)tord[tm];                                                        // wide tiles first (see the kernel's prologue)
     int lo = 0, hi = p.experts;                                                          // largest e with tb[e] <= tm (empty experts repeat a value)
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
         if (p.tb[mid] <= (uint32_t)tm) lo = mid; else hi = mid;
     }
-    it.m0 = (int)(p.off[lo] + ((uint32_t)tm - p.tb[lo]) * (uint32_t)(128 * p.msub));
-    it.m_end = (int)p.off[lo + 1];
-    it.nsub = min(p.msub, (it.m_end - it.m0 + 127) >> 7);                                // a segment tail of up to 128 rows runs one block
-    it.b_rt0 = (lo * p.n + it.n0) >> 4;
+    it.m0 = (int)(p.off[lo] + ((uint32_t)tm - p.tb[lo]) * (uint32_t)p.mt);
+    it.m_end = min((int)p.off[lo + 1], it.m0 + p.mt);
+    it.nn = PAIR ? (it.m_end - it.m0 + 31) & ~31 : (it.m_end - it.m0 + 15) & ~15;
+    it.rt0 = (lo * p.n + it.n0) >> 4;
     if (p.gs) it.gscale = p.gs[lo];
     if (p.gsb) it.gscale_b = p.gsb[lo];
     return it;
@@ -126,7 +149,6 @@ __device__ __forceinline__ uint32_t ldg16s(const uint8_t* p) {
     asm volatile("ld.global.nc.L1::no_allocate.u16 %0, [%1];" : "=h"(v) : "l"(p));
     return v;
 }
-__device__ __forceinline__ void sts64(uint32_t a, uint32_t x, uint32_t y) { asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y) : "memory"); }
 __device__ __forceinline__ void sts128(uint32_t a, uint4 v) { asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory"); }
 
 __device__ __forceinline__ uint32_t h2_sub(uint32_t a, uint32_t b) {
@@ -439,20 +461,6 @@ __device__ __forceinline__ void kq_compute_quarter(const KqTile<FMT>& tr, uint32
         }
     }
 }
-
-// The quarter's registers into the B stage. dst_g / dst_h: this lane's row addresses (8 (t & 1) already added). Under the 128-byte swizzle the 16-byte chunk of
-// slice i sits at ((2 i + (t >> 1)) ^ g) * 16, and the 16 lanes an 8-byte store serves together have only four values of g: if all of them stored the same slice they
-// would cover 4 distinct chunks (two-way bank conflict). So in step k the lanes with odd g store slice k ^ 2 instead of slice k: the 16 lanes then cover all 8
-// chunks of their rows and every store is conflict-free. cxs[k] is the swizzled offset of the slice this lane stores in step k.
-__device__ __forceinline__ void kq_store_quarter(uint32_t dst_g, uint32_t dst_h, const uint32_t (&cxs)[4], bool odd, const uint32_t (&r)[16]) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int a = 4 * k, b = 4 * (k ^ 2);
-        sts64(dst_g + cxs[k], odd ? r[b] : r[a], odd ? r[b + 1] : r[a + 1]);
-        sts64(dst_h + cxs[k], odd ? r[b + 2] : r[a + 2], odd ? r[b + 3] : r[a + 3]);
-    }
-}
-
 // After quarter P of a tile has been computed, the registers it alone used are refilled from the next tile (in place: one register set, every unit is requested a
 // whole tile ahead of its next use). Units shared by two quarters are refilled after the second one.
 template <int FMT, int P>
@@ -523,49 +531,125 @@ __device__ __forceinline__ void kq_refill_scales(const uint8_t* tile, int lane, 
     }
 }
 
+// ------------------------------------------------------------------------------------------------ tensor-memory and matrix-transpose building blocks
+// D[tmem] (+)= A[tmem] * B[smem]^T, issued by one thread
+template <bool PAIR>
+__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    if constexpr (PAIR)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+            : "memory");
+}
+// 16 lanes x 32 columns: repeat i covers columns 8 i .. 8 i + 7; lane (g, t): registers 4 i, 4 i + 1 = row g, columns 2 t, 2 t + 1; 4 i + 2, 4 i + 3 = row g + 8
+__device__ __forceinline__ void tmem_st_16x256b_x4(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
+                 "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
+                   "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                 : "r"(taddr)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// four 8 x 8 matrices of 16-bit elements, transposed: lane l gives the address of the 16 bytes that receive column l & 7 of matrix l >> 3
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+// a bounded wait of the whole warp whose answer is a vote, so that what depends on it stays uniform
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_fast(bar, parity)) != 0; }
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void epilogue_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }      // the four epilogue warps
+__device__ __forceinline__ uint32_t pack_sat(uint32_t a, uint32_t b, float s) {
+    __half2 h = sat_half2(__uint_as_float(a) * s, __uint_as_float(b) * s);
+    return *reinterpret_cast<uint32_t*>(&h);
+}
 
-template <int FMT>
+// The tiles of one decoder warp over all its items: every second T16 tile (parity kp of the CTA's running tile count) of one row tile.
+template <int TB, bool PAIR>
+struct KqWalk {
+    const uint8_t* ptr;         // current tile
+    int t, kb, ntb, base;       // item, block inside the item's range, blocks of the range, parity of the tiles before the item
+    bool ok;
+
+    __device__ __forceinline__ void enter(const KqParams& p, int num_items, int stride, uint32_t rank, const uint16_t* tord, int kp, int q, int half) {
+        ok = false;
+        for (; t < num_items; t += stride) {
+            const KqItem it = kq_item<PAIR>(p, t, rank, tord);
+            if (!it.valid) return;                                                     // grouped form: all items behind it are invalid too
+            ntb = it.ntb, kb = kp ^ base;
+            if (kb < ntb) {
+                const int rt = min(it.rt0 + (p.glu ? q : 2 * q + half), p.rt_total - 1);
+                ptr = ((p.glu && half) ? p.t16b : p.t16) + ((size_t)rt * (size_t)p.nb + (size_t)(it.tb0 + kb)) * TB;
+                ok = true;
+                return;
+            }
+            base ^= ntb & 1;
+        }
+    }
+    __device__ __forceinline__ void advance(const KqParams& p, int num_items, int stride, uint32_t rank, const uint16_t* tord, int kp, int q, int half) {
+        kb += 2;
+        if (kb < ntb) {
+            ptr += 2 * TB;
+            return;
+        }
+        base ^= ntb & 1, t += stride;
+        enter(p, num_items, stride, rank, tord, kp, q, half);
+    }
+};
+
+template <int FMT, bool PAIR>
 __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_kq_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ KqOutMaps outs, const KqParams p,
                                                                  const int num_items) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     constexpr int TB = kyb_tile_bytes(FMT);
-    const uint32_t a_bytes = (uint32_t)p.msub * KQ_A_SUB, stage_bytes = a_bytes + KQ_B_BYTES;
-    const int STAGES = p.stages;
+    const uint32_t BS = (uint32_t)p.bstages;                                         // 4 or 2
     const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t scr0 = smem0 + (uint32_t)STAGES * stage_bytes;
-    const uint32_t stg0 = scr0 + KQ_DW * KQ_SCR;                                    // epilogue staging, 4 warps
-    const uint32_t stg_bytes = p.wide ? 2 * KQ_STG : KQ_STG;
-    const uint32_t bars = stg0 + 4 * stg_bytes;                                     // full[STAGES], empty[STAGES], acc_full[2], acc_empty[2], tmem slot
-    const uint32_t full0 = bars, empty0 = bars + 8 * STAGES, accf0 = bars + 16 * STAGES, acce0 = accf0 + 16, tmem_slot = acce0 + 16;
+    const uint32_t stg0 = smem0 + (uint32_t)BS * p.bstage_bytes;
+    const uint32_t scr0 = stg0 + 2 * KQ_STG;
+    const uint32_t bars = scr0 + KQ_DW * KQ_SCR;                                    // full[4], empty[4], acc_full[2], acc_empty[2], tmem slot
+    const uint32_t full0 = bars, empty0 = bars + 32, accf0 = bars + 64, acce0 = bars + 80, tmem_slot = bars + 96;
+    const uint32_t tord_a = bars + 112;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = PAIR ? cluster_rank() : 0u;
+    const int first = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, stride = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
     constexpr uint32_t TMEM_COLS = 512;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) mbar_init_a(full0 + 8 * s, KQ_DW + 1), mbar_init_a(empty0 + 8 * s, 1);
-        for (int a = 0; a < 2; ++a) mbar_init_a(accf0 + 8 * a, 1), mbar_init_a(acce0 + 8 * a, 4);
+        for (int s = 0; s < KQ_SA; ++s) mbar_init_a(full0 + 8 * s, (PAIR ? 2 : 1) * KQ_DW / 2 + 1), mbar_init_a(empty0 + 8 * s, 1);
+        for (int a = 0; a < 2; ++a) mbar_init_a(accf0 + 8 * a, 1), mbar_init_a(acce0 + 8 * a, PAIR ? 8 : 4);
         mbar_fence_init();
         prefetch_tmap(&tma_a);
     }
-    if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
-    // Grouped form with two-block items: a tile with more than 128 rows costs about 1.5 times a tile with fewer (eight MMAs per stage instead of four), and items go
-    // to the CTAs round-robin, so the tiles are renumbered with the two-block ones first: every CTA then gets the same number of them (+-1) instead of a random
-    // share. Warp 2 builds the table (two-block tiles from the front, the others from the back) from the segment offsets; more tiles than the table holds keep
-    // their order.
+    if (warp == 1) {
+        if constexpr (PAIR) tmem_alloc_pair(tmem_slot, TMEM_COLS);
+        else tmem_alloc(tmem_slot, TMEM_COLS);
+    }
+    // Grouped form with items of up to 256 rows: a tile with more than 128 rows costs more than one with fewer, and items go to the CTAs round-robin, so the tiles
+    // are renumbered with the wide ones first: every CTA then gets the same number of them (+-1) instead of a random share. Warp 2 builds the table (wide tiles from
+    // the front, the others from the back) from the segment offsets; more tiles than the table holds keep their order.
     const uint16_t* tord = nullptr;
-    if (p.tb && p.msub == 2) {
+    if (p.tb && p.mt == 256) {
         const uint32_t total = p.tb[p.experts];
         if (total <= (uint32_t)KQ_TORD) {
-            uint16_t* tw = reinterpret_cast<uint16_t*>(smem_raw + (tmem_slot + 16 - smem_u32(smem_raw)));
+            uint16_t* tw = reinterpret_cast<uint16_t*>(smem_raw + (tord_a - smem_u32(smem_raw)));
             tord = tw;
             if (warp == 2) {
                 uint32_t front = 0, back = total;
                 for (int e0 = 0; e0 < p.experts; e0 += 32) {
                     const int e = e0 + lane;
-                    uint32_t two = 0, one = 0, first = 0;
+                    uint32_t two = 0, one = 0, first_tile = 0;
                     if (e < p.experts) {
                         const uint32_t rows = p.off[e + 1] - p.off[e], nt = (rows + 255u) >> 8;
-                        first = p.tb[e];
+                        first_tile = p.tb[e];
                         one = (nt && rows - 256u * (nt - 1u) <= 128u) ? 1u : 0u;
                         two = nt - one;
                     }
@@ -575,294 +659,313 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_kq_kernel(const __grid_con
                         const uint32_t ua = __shfl_up_sync(0xffffffffu, a, d), ub = __shfl_up_sync(0xffffffffu, b, d);
                         if (lane >= d) a += ua, b += ub;
                     }
-                    for (uint32_t i = 0; i < two; ++i) tw[front + a - two + i] = (uint16_t)(first + i);
-                    if (one) tw[back - b] = (uint16_t)(first + two);
+                    for (uint32_t i = 0; i < two; ++i) tw[front + a - two + i] = (uint16_t)(first_tile + i);
+                    if (one) tw[back - b] = (uint16_t)(first_tile + two);
                     front += __shfl_sync(0xffffffffu, a, 31), back -= __shfl_sync(0xffffffffu, b, 31);
                 }
             }
         }
     }
     tc_fence_before();
-    __syncthreads();
+    if constexpr (PAIR) cluster_sync_all();                                         // both CTAs' barriers exist before either signals the other
+    else __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = lds32(tmem_slot);
     bool failed = false;
 
     if (warp == 0) {
-        // ---- TMA producer: activation tiles
-        if (elect_one()) {
-            uint32_t parity = 1;                                                    // a fresh barrier passes a wait on the previous phase
-            int s = 0;
-            for (int t = blockIdx.x; t < num_items && !failed; t += gridDim.x) {
-                const KqItem it = kq_item(p, t, tord);
-                if (!it.valid) continue;
-                for (int kb = 4 * it.tb0; kb < 4 * (it.tb0 + it.ntb) && !failed; ++kb) {
-                    if (!mbar_wait_fast(empty0 + 8 * s, parity)) failed = true;
-                    const uint32_t a_dst = smem0 + s * stage_bytes;
-                    mbar_expect_tx_a(full0 + 8 * s, (uint32_t)it.nsub * KQ_A_SUB);
-                    for (int sub = 0; sub < it.nsub; ++sub) tma_load_2d(a_dst + sub * KQ_A_SUB, &tma_a, kb * KQ_BK, it.m0 + sub * 128, full0 + 8 * s);
-                    if (++s == STAGES) s = 0, parity ^= 1u;
+        // ---- TMA producer: activation boxes. Stage i of the run uses barrier full[i % 4] (with the decoders of that stage) and shared-memory stage i % BS, which is free
+        // once the MMAs of stage i - BS are done. By pairs each CTA loads its half of the item's rows and all bytes complete on the leader's barrier.
+        // This loop and the MMA issuer's are executed by the whole warp, their conditions are warp votes and one elected lane issues, so that addresses and
+        // descriptors stay in uniform registers (inside the elected lane's branch every operand of every MMA went through vector registers: 75 clocks per MMA). A
+        // stage is 128 inputs because the instructions around a stage (waits, expect_tx, commit: 200-250 clocks in either warp) are paid per stage.
+        const bool lead = elect_one();
+        const uint32_t fullr0 = PAIR ? map_to_rank(full0, 0) : full0;
+        uint32_t i = 0;
+        bool ok = true;
+        for (int t = first; t < num_items && ok; t += stride) {
+            const KqItem it = kq_item<PAIR>(p, t, rank, tord);
+            if (!it.valid) break;
+            const uint32_t rows = __reduce_max_sync(0xffffffffu, (uint32_t)it.nn) >> (PAIR ? 1 : 0), boxes = (rows + p.box_rows - 1u) / p.box_rows;
+            const uint32_t end = i + 2u * __reduce_max_sync(0xffffffffu, (uint32_t)it.ntb), bytes = (PAIR ? 4u : 2u) * boxes * p.box_rows * 128u;
+            const int y0 = __reduce_max_sync(0xffffffffu, it.m0) + (PAIR ? (int)(rank * rows) : 0);
+            int x = __reduce_max_sync(0xffffffffu, it.tb0) * 256;
+            for (; i < end && ok; ++i, x += KQ_BK) {
+                if (i >= BS) ok = mbar_wait_warp(empty0 + 8 * ((i - BS) & 3u), ((i - BS) >> 2) & 1u);
+                if (lead) {
+                    const uint32_t dst = smem0 + (i & (BS - 1u)) * p.bstage_bytes, bar = fullr0 + 8 * (i & 3u);
+                    if (rank == 0) mbar_expect_tx_a(full0 + 8 * (i & 3u), bytes);
+                    for (uint32_t b = 0; b < boxes; ++b)
+#pragma unroll
+                        for (uint32_t h = 0; h < 2; ++h) {
+                            const uint32_t d = dst + h * (p.bstage_bytes >> 1) + b * p.box_rows * 128u;
+                            if constexpr (PAIR) tma_load_2d_pair(d, &tma_a, x + 64 * (int)h, y0 + (int)(p.box_rows * b), bar);
+                            else tma_load_2d(d, &tma_a, x + 64 * (int)h, y0 + (int)(p.box_rows * b), bar);
+                        }
                 }
+                __syncwarp();
             }
         }
+        failed = !ok;
     } else if (warp == 1) {
-        // ---- MMA issuer
-        if (elect_one()) {
-            constexpr uint32_t idesc = umma_idesc_f16(128, KQ_BN);
-            uint32_t parity = 0;
-            int s = 0;
-            uint32_t cnt = 0;                                                       // accumulators used so far: number cnt lives in slot cnt & 1
-            for (int t = blockIdx.x; t < num_items && !failed; t += gridDim.x) {
-                const KqItem it = kq_item(p, t, tord);
-                if (!it.valid) continue;
-                // the epilogue must have drained an accumulator before the first MMA into it; the second block's accumulator is waited for only when its first MMA
-                // is due, so the first stage of this item overlaps the tail of the previous item's epilogue
-                if (!mbar_wait_fast(acce0 + 8 * (cnt & 1u), ((cnt >> 1) & 1u) ^ 1u)) failed = true;
-                tc_fence_after();
-                for (int kb = 0; kb < 4 * it.ntb && !failed; ++kb) {
-                    if (!mbar_wait_fast(full0 + 8 * s, parity)) failed = true;
+        // ---- MMA issuer (by pairs: the leader's)
+        if (rank == 0) {
+            const bool lead = elect_one();
+            uint32_t i = 0, slot = 0, uses = 0;                                     // bit a of uses = parity of the uses of accumulator slot a
+            const uint64_t desc0 = umma_desc_sw128(smem0);
+            const uint32_t dstage = p.bstage_bytes >> 4, dhalf = p.bstage_bytes >> 5;
+            bool ok = true;
+            for (int t = first; t < num_items && ok; t += stride) {
+                const KqItem it = kq_item<PAIR>(p, t, rank, tord);
+                if (!it.valid) break;
+                const uint32_t nn = __reduce_max_sync(0xffffffffu, (uint32_t)it.nn), end = i + 2u * __reduce_max_sync(0xffffffffu, (uint32_t)it.ntb);
+                const uint32_t idesc = umma_idesc_f16(PAIR ? 256 : 128, (int)nn);
+                if (nn > 128u) slot = 0;                                            // a wide item takes both slots
+                const uint32_t tmem_d = tmem_base + slot * 128u, used = nn > 128u ? 3u : 1u << slot;
+                // the epilogue must have drained an accumulator before the first MMA into it
+                ok = mbar_wait_warp(acce0 + 8 * slot, ((uses >> slot) & 1u) ^ 1u);
+                if (nn > 128u && ok) ok = mbar_wait_warp(acce0 + 8, ((uses >> 1) & 1u) ^ 1u);
+                for (uint32_t acc = 0; i < end && ok; ++i, acc = 1) {
+                    ok = mbar_wait_warp(full0 + 8 * (i & 3u), (i >> 2) & 1u);
                     tc_fence_after();
-                    const uint32_t a_src = smem0 + s * stage_bytes;
-                    const uint64_t bdesc = umma_desc_sw128(a_src + a_bytes);
-                    for (int sub = 0; sub < it.nsub; ++sub) {
-                        const uint64_t adesc = umma_desc_sw128(a_src + sub * KQ_A_SUB);
-                        const uint32_t tmem_d = tmem_base + (uint32_t)(((cnt + sub) & 1u) * KQ_BN);
-                        if (kb == 0 && sub) {
-                            if (!mbar_wait_fast(acce0 + 8 * ((cnt + 1u) & 1u), (((cnt + 1u) >> 1) & 1u) ^ 1u)) failed = true;
-                            tc_fence_after();
-                        }
+                    const uint32_t tmem_a = tmem_base + KQ_COL_A + 64u * (i & 3u);
+                    const uint64_t bd = desc0 + (i & (BS - 1u)) * dstage;
+                    if (lead) {
 #pragma unroll
-                        for (int kk = 0; kk < KQ_BK / 16; ++kk) umma_f16(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (kb | kk) != 0);
+                        for (int kk = 0; kk < KQ_BK / 16; ++kk) umma_f16_ta<PAIR>(tmem_d, tmem_a + 8 * kk, bd + (kk >= 4 ? dhalf : 0u) + 2 * (kk & 3), idesc, kk ? 1u : acc);
+                        if constexpr (PAIR) umma_commit_pair(empty0 + 8 * (i & 3u));    // the weight stage and the activation stage are free once these MMAs have read them
+                        else umma_commit(empty0 + 8 * (i & 3u));
                     }
-                    umma_commit(empty0 + 8 * s);                                    // stage free once these MMAs have read it
-                    if (++s == STAGES) s = 0, parity ^= 1u;
+                    __syncwarp();
                 }
-                for (int sub = 0; sub < it.nsub; ++sub) umma_commit(accf0 + 8 * ((cnt + sub) & 1u));
-                cnt += (uint32_t)it.nsub;
+                if (lead) {
+                    for (uint32_t a = 0; a < 2; ++a)
+                        if (used & (1u << a)) {
+                            if constexpr (PAIR) umma_commit_pair(accf0 + 8 * a);
+                            else umma_commit(accf0 + 8 * a);
+                        }
+                }
+                __syncwarp();
+                uses ^= used, slot ^= nn > 128u ? 0u : 1u;
             }
+            failed = !ok;
         }
     } else if (warp < 6) {
-        // ---- epilogue: warp w may touch TMEM lanes [32 (w % 4), 32 (w % 4) + 32)
+        // ---- epilogue: warp w may touch TMEM lanes [32 (w % 4), 32 (w % 4) + 32) = outputs n0 + 32 q ..
         const int q = warp & 3;
-        uint32_t cnt = 0;
-        for (int t = blockIdx.x; t < num_items; t += gridDim.x) {
-            const KqItem it = kq_item(p, t, tord);
-            if (!it.valid) continue;
-            for (int sub = 0; sub < it.nsub; ++sub, ++cnt) {
-                const uint32_t slot = cnt & 1u;
-                if (!mbar_wait_fast(accf0 + 8 * slot, (cnt >> 1) & 1u)) failed = true;
+        const uint32_t acce = PAIR ? map_to_rank(acce0, 0) : acce0;
+        const uint32_t tq = tmem_base + ((uint32_t)(q * 32) << 16);
+        uint32_t next = 0, uses = 0, ch = 0;                                          // accumulator slots as the MMA issuer deals them; staged 32-row chunks so far
+        for (int t = first; t < num_items; t += stride) {
+            const KqItem it = kq_item<PAIR>(p, t, rank, tord);
+            if (!it.valid) break;
+            const int nsub = it.nn > 128 ? 2 : 1;
+            for (int sub = 0; sub < nsub; ++sub) {
+                const uint32_t slot = nsub == 2 ? (uint32_t)sub : next;
+                if (!failed && !mbar_wait_fast(accf0 + 8 * slot, (uses >> slot) & 1u)) failed = true;
+                uses ^= 1u << slot, next = slot ^ 1u;
                 tc_fence_after();
-                const float gscale = it.gscale;
-                if (p.part) {
-                    // ---- split-k: this range's accumulator as it is (fp32) through the staged tiled stores; the tensor map covers part as 16-bit pairs, so a step of
-                    // 32 rows x 16 fp32 columns is the same 32 x 64-byte box as a step of fp16 outputs. Rows past m land in the padding rows of the range.
-                    const uint32_t stg = stg0 + (uint32_t)q * stg_bytes;
-                    const int row0 = it.sp * p.mpad + it.m0 + sub * 128 + q * 32;
-#pragma unroll 1
-                    for (int c = 0; c < KQ_BN; c += 32) {
+                const int cols = min(it.nn - 128 * sub, 128);
+                for (int c = 0; c < cols; c += 32) {
+                    const int row0 = it.m0 + 128 * sub + c;
+                    const bool last = c + 32 >= cols;
+                    if (p.part) {
+                        // ---- split-k: this range's accumulator as it is (fp32): every column is one activation row, a warp's 32 outputs are 128 contiguous bytes
                         uint32_t v[32];
-                        tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + slot * KQ_BN + (uint32_t)c, v);
+                        tmem_ld_32x32(tq + slot * 128u + (uint32_t)c, v);
                         tmem_ld_wait();
-                        uint32_t w[16];
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) w[j] = v[j];
-                        epilogue_stage_store(outs, 1, stg, lane, w, 2 * (it.n0 + c), row0, !failed);
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) w[j] = v[16 + j];
-                        epilogue_stage_store(outs, 1, stg, lane, w, 2 * (it.n0 + c + 16), row0, !failed);
-                    }
-                } else if (p.tma_out) {
-                    // ---- staged tiled stores: 32 rows x 32 columns per step go to shared memory (64-byte swizzle, conflict-free 16-byte stores) and leave as one bulk
-                    // tensor store per receiving rank: full 64-byte row segments on the wire, rows / columns past the matrix are dropped by the tensor map
-                    const uint32_t stg = stg0 + (uint32_t)q * stg_bytes;
-                    const int row0 = it.m0 + sub * 128 + q * 32;
-#pragma unroll 1
-                    for (int c = 0; c < KQ_BN; c += 32) {
-                        uint32_t v[32];
-                        tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + slot * KQ_BN + (uint32_t)c, v);
-                        tmem_ld_wait();
-                        uint32_t w[16];
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            __half2 h = sat_half2(__uint_as_float(v[2 * j]) * gscale, __uint_as_float(v[2 * j + 1]) * gscale);
-                            w[j] = *reinterpret_cast<uint32_t*>(&h);
-                        }
-                        if (p.wide)
-                            epilogue_stage_store_wide(outs, p.nout, stg, lane, w, (c >> 5) & 1, p.col0 + it.n0 + (c & ~63), row0,
-                                                      !failed && row0 < it.m_end && it.n0 + (c & ~63) < p.n);
-                        else
-                            epilogue_stage_store(outs, p.nout, stg, lane, w, p.col0 + it.n0 + c, row0, !failed && row0 < it.m_end && it.n0 + c < p.n);
-                    }
-                } else if (p.tb && (p.ldd & 7) == 0 && ((uintptr_t)p.d[0] & 15) == 0) {
-                    // ---- grouped form: rows end inside a tile or are scattered, so no tensor map fits. A step of 32 rows x 32 columns is transposed through the warp's
-                    // staging buffer: every store instruction then writes 64-byte row segments (8 rows x 4 lanes) instead of 16 bytes of each of 32 rows
-                    const uint32_t stg = stg0 + (uint32_t)q * stg_bytes;
-                    const int row0 = it.m0 + sub * 128 + q * 32, row = row0 + lane;
-                    const uint32_t orow = (p.row_map && row < it.m_end) ? p.row_map[row] : (uint32_t)row;
-                    __half* dst[4];
-                    bool live[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int rr = 8 * i + (lane >> 2);
-                        const uint32_t o = __shfl_sync(0xffffffffu, orow, rr);
-                        live[i] = row0 + rr < it.m_end && !failed;
-                        dst[i] = p.d[0] + (size_t)o * p.ldd + it.n0 + 8 * (lane & 3);
-                    }
-#pragma unroll 1
-                    for (int c = 0; c < (p.glu ? KQ_BN / 2 : KQ_BN); c += 32) {
-                        uint32_t v[32], w[16];
-                        tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + slot * KQ_BN + (uint32_t)c, v);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            __half2 h = sat_half2(__uint_as_float(v[2 * i]) * gscale, __uint_as_float(v[2 * i + 1]) * gscale);
-                            w[i] = *reinterpret_cast<uint32_t*>(&h);
-                        }
-                        if (p.glu) {
-                            // w holds the gate products rounded to fp16 (what the reference's two-launch form would have stored); the up products of the same
-                            // output columns sit 128 accumulator columns further
-                            tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + slot * KQ_BN + (uint32_t)(KQ_BN / 2 + c), v);
-                            tmem_ld_wait();
-                            const float gsb = it.gscale_b, lim = p.limit;
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) {
-                                const __half2 a2 = *reinterpret_cast<__half2*>(&w[i]);
-                                float a0 = __low2float(a2), a1 = __high2float(a2);
-                                float b0 = __half2float(sat_half(__uint_as_float(v[2 * i]) * gsb)), b1 = __half2float(sat_half(__uint_as_float(v[2 * i + 1]) * gsb));
-                                if (lim > 0.f) a0 = fminf(a0, lim), a1 = fminf(a1, lim), b0 = fminf(fmaxf(b0, -lim), lim), b1 = fminf(fmaxf(b1, -lim), lim);
-                                __half2 h = sat_half2(a0 * (1.0f / (1.0f + expf(-a0))) * b0, a1 * (1.0f / (1.0f + expf(-a1))) * b1);
-                                w[i] = *reinterpret_cast<uint32_t*>(&h);
+                        if (last) {
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) {
+                                if constexpr (PAIR) mbar_arrive_cluster(acce + 8 * slot);
+                                else mbar_arrive_a(acce + 8 * slot);
                             }
                         }
-                        __syncwarp();                                                  // the previous step's reads of the staging buffer are done
+                        float* dst = p.part + ((size_t)it.sp * (size_t)p.mpad + (size_t)row0) * (size_t)p.ldp + it.n0 + 32 * q + lane;
 #pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            sts128(stg + (uint32_t)lane * 64u + (uint32_t)((j ^ ((lane >> 1) & 3)) << 4), make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]));
-                        __syncwarp();
+                        for (int j = 0; j < 32; ++j)
+                            if (row0 + j < it.m_end && !failed) dst[(size_t)j * (size_t)p.ldp] = __uint_as_float(v[j]);
+                        continue;
+                    }
+                    // rows of the staged chunk that this warp will store (row stores): 8 rows, 16 (gated pair: 8) lanes of 16 bytes each
+                    uint32_t orow[4];
+                    if (!p.tma_out) {
+                        const int per = p.glu ? 4 : 2;                                  // rows per store instruction
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
-                            const int rr = 8 * i + (lane >> 2);
-                            const uint4 o = lds128(stg + (uint32_t)rr * 64u + (uint32_t)(((lane & 3) ^ ((rr >> 1) & 3)) << 4));
-                            if (live[i]) *reinterpret_cast<uint4*>(dst[i] + c) = o;
+                            const int row = row0 + 8 * q + per * i + (p.glu ? lane >> 3 : lane >> 4);
+                            orow[i] = (uint32_t)row;
+                            if (p.row_map && i < 8 / per && row < it.m_end) orow[i] = p.row_map[row];
                         }
                     }
-                } else {
-                const int row = it.m0 + sub * 128 + q * 32 + lane;
-                const size_t orow = (p.row_map && row < it.m_end) ? (size_t)p.row_map[row] : (size_t)row;
-                const size_t doff = orow * p.ldd + it.n0;
-#pragma unroll 1
-                for (int c = 0; c < KQ_BN; c += 32) {
-                    uint32_t v[32];
-                    tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + slot * KQ_BN + (uint32_t)c, v);
+                    uint32_t va[16], vb[16];                                            // outputs 32 q + g, + 8 and 32 q + 16 + g, + 8, activation rows 8 i + 2 t, + 1
+                    tmem_ld_16x256b_x4(tq + slot * 128u + (uint32_t)c, va);
+                    tmem_ld_16x256b_x4(tq + (16u << 16) + slot * 128u + (uint32_t)c, vb);
                     tmem_ld_wait();
-                    if (row < it.m_end && !failed) {
-                        if (it.n0 + c + 32 <= p.n && (p.ldd & 7) == 0) {
+                    if (last) {                                                         // this warp has read its quarter of the accumulator
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) {
+                            if constexpr (PAIR) mbar_arrive_cluster(acce + 8 * slot);
+                            else mbar_arrive_a(acce + 8 * slot);
+                        }
+                    }
+                    const uint32_t stg = stg0 + (ch & 1u) * KQ_STG;
+                    if (p.glu) {
+                        // va holds the gate products, vb the up products of the same 16 outputs; both are rounded to fp16 (what separate launches would have stored)
+                        const float ga = it.gscale, gb = it.gscale_b, lim = p.limit;
+                        uint32_t w[8];
 #pragma unroll
-                            for (int j = 0; j < 32; j += 8) {
-                                uint4 o;
-                                __half2 h0 = sat_half2(__uint_as_float(v[j]) * gscale, __uint_as_float(v[j + 1]) * gscale);
-                                __half2 h1 = sat_half2(__uint_as_float(v[j + 2]) * gscale, __uint_as_float(v[j + 3]) * gscale);
-                                __half2 h2 = sat_half2(__uint_as_float(v[j + 4]) * gscale, __uint_as_float(v[j + 5]) * gscale);
-                                __half2 h3 = sat_half2(__uint_as_float(v[j + 6]) * gscale, __uint_as_float(v[j + 7]) * gscale);
-                                o.x = *reinterpret_cast<uint32_t*>(&h0), o.y = *reinterpret_cast<uint32_t*>(&h1), o.z = *reinterpret_cast<uint32_t*>(&h2), o.w = *reinterpret_cast<uint32_t*>(&h3);
-                                for (int pr = 0; pr < p.nout; ++pr) *reinterpret_cast<uint4*>(p.d[pr] + doff + c + j) = o;
+                        for (int i = 0; i < 8; ++i) {
+                            __half2 a2 = sat_half2(__uint_as_float(va[2 * i]) * ga, __uint_as_float(va[2 * i + 1]) * ga);
+                            __half2 b2 = sat_half2(__uint_as_float(vb[2 * i]) * gb, __uint_as_float(vb[2 * i + 1]) * gb);
+                            float a0 = __low2float(a2), a1 = __high2float(a2), b0 = __low2float(b2), b1 = __high2float(b2);
+                            if (lim > 0.f) a0 = fminf(a0, lim), a1 = fminf(a1, lim), b0 = fminf(fmaxf(b0, -lim), lim), b1 = fminf(fmaxf(b1, -lim), lim);
+                            __half2 h = sat_half2(a0 * (1.0f / (1.0f + expf(-a0))) * b0, a1 * (1.0f / (1.0f + expf(-a1))) * b1);
+                            w[i] = *reinterpret_cast<uint32_t*>(&h);
+                        }
+#pragma unroll
+                        for (int i = 0; i < 4; i += 2) {                               // matrices (i, outputs 0-7), (i, 8-15), (i + 1, 0-7), (i + 1, 8-15)
+                            const uint32_t row = 8u * (i + (lane >> 4)) + (lane & 7), c16 = 2u * q + ((lane >> 3) & 1);
+                            stmatrix_x4_trans(stg + row * 128u + ((c16 ^ (row & 7u)) << 4), w[2 * i], w[2 * i + 1], w[2 * i + 2], w[2 * i + 3]);
+                        }
+                    } else {
+                        const float gscale = it.gscale;
+                        const uint32_t c16 = 4u * (q & 1) + (lane >> 3), half_tile = stg + (uint32_t)(q >> 1) * 4096u + ((c16 ^ (lane & 7)) << 4) + (lane & 7) * 128u;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)                                    // matrices: outputs 0-7, 8-15, 16-23, 24-31 of the warp, activation rows 8 i .. 8 i + 7
+                            stmatrix_x4_trans(half_tile + 1024u * i, pack_sat(va[4 * i], va[4 * i + 1], gscale), pack_sat(va[4 * i + 2], va[4 * i + 3], gscale),
+                                              pack_sat(vb[4 * i], vb[4 * i + 1], gscale), pack_sat(vb[4 * i + 2], vb[4 * i + 3], gscale));
+                    }
+                    if (p.tma_out) {
+                        fence_proxy_async_smem();
+                        // the other staging tile is free for the next chunk once the stores issued from it have read it: waited for before the barrier
+                        if (warp == 2 && lane == 0) tma_store_wait_read();
+                        epilogue_barrier();
+                        if (warp == 2 && lane == 0) {
+                            if (!failed && row0 < it.m_end)
+                                for (int pr = 0; pr < p.nout; ++pr)
+                                    for (int h = 0; h < 2; ++h)
+                                        if (it.n0 + 64 * h < p.n) tma_store_2d(&outs.m[pr], stg + 4096u * h, p.col0 + it.n0 + 64 * h, row0);
+                            tma_store_commit();
+                        }
+                    } else {
+                        epilogue_barrier();
+                        if (p.glu) {
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) {
+                                const uint32_t rr = 8u * q + 4u * i + (lane >> 3), c16 = lane & 7;
+                                const uint4 o = lds128(stg + rr * 128u + ((c16 ^ (rr & 7u)) << 4));
+                                if (row0 + (int)rr < it.m_end && !failed) *reinterpret_cast<uint4*>(p.d[0] + (size_t)orow[i] * p.ldd + it.n0 + 8 * c16) = o;
                             }
                         } else {
 #pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                if (it.n0 + c + j < p.n)
-                                    for (int pr = 0; pr < p.nout; ++pr) p.d[pr][doff + c + j] = sat_half(__uint_as_float(v[j]) * gscale);
+                            for (int i = 0; i < 4; ++i) {
+                                const uint32_t rr = 8u * q + 2u * i + (lane >> 4), c16 = lane & 15;
+                                const uint4 o = lds128(stg + (c16 >> 3) * 4096u + rr * 128u + (((c16 & 7u) ^ (rr & 7u)) << 4));
+                                const int col = it.n0 + 8 * (int)c16;
+                                if (row0 + (int)rr < it.m_end && !failed) {
+                                    if (p.vec_out && col + 8 <= p.n) {
+                                        for (int pr = 0; pr < p.nout; ++pr) *reinterpret_cast<uint4*>(p.d[pr] + (size_t)orow[i] * p.ldd + col) = o;
+                                    } else {
+                                        const uint32_t ow[4] = {o.x, o.y, o.z, o.w};
+                                        for (int pr = 0; pr < p.nout; ++pr)
+#pragma unroll
+                                            for (int j = 0; j < 8; ++j)
+                                                if (col + j < p.n) p.d[pr][(size_t)orow[i] * p.ldd + col + j] = __ushort_as_half((unsigned short)(ow[j >> 1] >> (16 * (j & 1))));
+                                    }
+                                }
+                            }
                         }
                     }
+                    ++ch;
                 }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_a(acce0 + 8 * slot);                       // this warp has read its quarter of the accumulator
             }
         }
     } else {
         // ---- decoders
-        const int dw = warp - 6, g = lane >> 2, tq = lane & 3;
+        const int dw = warp - 6, q = warp & 3, half = (dw >> 2) & 1, kp = dw >> 3;
         const uint32_t scr = scr0 + dw * KQ_SCR;
-        // rows 16 dw + g and 16 dw + g + 8 of the B tile: 128-byte rows in 8-row groups of 1024 bytes, 16-byte chunks XOR-swizzled with the row number (row & 7 = g)
-        const uint32_t row_off = (uint32_t)(2 * dw) * 1024u + (uint32_t)g * 128u + 8u * (uint32_t)(tq & 1);
-        const bool odd = (g & 1) != 0;
-        uint32_t cx[4];                                                              // offset of the slice this lane stores in step k (see kq_store_quarter)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) cx[i] = (uint32_t)(((2 * (i ^ (odd ? 2 : 0)) + (tq >> 1)) ^ g) * 16);
-        uint32_t parity = 1;
-        int s = 0;
-        for (int t = blockIdx.x; t < num_items && !failed; t += gridDim.x) {
-            const KqItem it = kq_item(p, t, tord);
-            if (!it.valid) continue;
-            const int rt = min(it.b_rt0 + (p.glu ? (dw & 7) : dw), p.rt_total - 1);      // gated pair: warps 0-7 decode the gate rows, 8-15 the same rows of the up stack
-            const uint8_t* tp = ((p.glu && dw >= 8) ? p.t16b : p.t16) + ((size_t)rt * (size_t)p.nb + (size_t)it.tb0) * TB;
-            const int nbk = it.ntb;                                                      // 256-input blocks of this item
-            // Software pipeline over the 64-input quarters: while the stores of quarter q drain into the stage (and before the proxy fence that publishes them), the
-            // registers of quarter q + 1 are computed, so the wait for a free stage, the scale loads and the arithmetic overlap the shared-memory traffic.
+        const uint32_t tw = tmem_base + ((uint32_t)(32 * q + 16 * half) << 16) + KQ_COL_A + 128u * (uint32_t)kp;   // this warp's 16 lanes, stages 2 kp and 2 kp + 1
+        const uint32_t full = (PAIR ? map_to_rank(full0, 0) : full0) + 16u * (uint32_t)kp, empty = empty0 + 16u * (uint32_t)kp;
+        KqWalk<TB, PAIR> wk;
+        wk.t = first, wk.base = 0;
+        wk.enter(p, num_items, stride, rank, tord, kp, q, half);
+        uint32_t parity = 1;                                                            // a fresh barrier passes a wait on the previous phase
+        bool more = wk.ok;
+        if (more) {
+            // Software pipeline over the 64-input quarters: while the tensor-memory store of quarter P is on its way, the registers of quarter P + 1 are computed; the
+            // wait for a free stage, the scale loads and the arithmetic overlap it.
             KqTile<FMT> tr;
             uint32_t r[16];
-            kq_load<FMT>(tp, lane, tr);
+            kq_load<FMT>(wk.ptr, lane, tr);
             kq_prep_scales<FMT>(tr, scr, lane);
             __syncwarp();
-            if (nbk > 1) kq_refill_scales<FMT>(tp + TB, lane, tr);
+            wk.advance(p, num_items, stride, rank, tord, kp, q, half);
+            if (wk.ok) kq_refill_scales<FMT>(wk.ptr, lane, tr);
             kq_compute_quarter<FMT, 0>(tr, scr, lane, r);
-            if (nbk > 1) kq_refill<FMT, 0>(tp + TB, lane, tr);
-#define KYB_KQ_PUBLISH()                                                                                          \
-    {                                                                                                             \
-        fence_proxy_async_smem();                                                                                 \
-        __syncwarp();                                                                                             \
-        if (lane == 0) mbar_arrive_a(full0 + 8 * s);                                                              \
-        if (++s == STAGES) s = 0, parity ^= 1u;                                                                   \
+            if (wk.ok) kq_refill<FMT, 0>(wk.ptr, lane, tr);
+#define KYB_KQ_WAIT(H)                                                               \
+    {                                                                                \
+        if (!mbar_wait_fast(empty + 8 * (H), parity)) failed = true;                 \
+        tc_fence_after();                                                            \
     }
-#define KYB_KQ_STORE()                                                                                            \
-    {                                                                                                             \
-        if (!mbar_wait_fast(empty0 + 8 * s, parity)) failed = true;                                               \
-        const uint32_t b_dst = smem0 + s * stage_bytes + a_bytes + row_off;                                       \
-        kq_store_quarter(b_dst, b_dst + 1024u, cx, odd, r);                                                       \
+#define KYB_KQ_PUBLISH(H)                                                            \
+    {                                                                                \
+        tmem_st_wait();                                                              \
+        tc_fence_before();                                                           \
+        __syncwarp();                                                                \
+        if (lane == 0) {                                                             \
+            if constexpr (PAIR) mbar_arrive_remote(full + 8 * (H));                  \
+            else mbar_arrive_a(full + 8 * (H));                                      \
+        }                                                                            \
     }
-            for (int kb = 0; kb < nbk && !failed; ++kb) {
-                const bool more = kb + 1 < nbk, more2 = kb + 2 < nbk;
-                const uint8_t* nx = tp + (size_t)(kb + 1) * TB;                      // the next tile, two tiles ahead for the units already consumed
-                KYB_KQ_STORE()
+            while (more && !failed) {
+                more = wk.ok;                                                           // wk is one tile ahead
+                KYB_KQ_WAIT(0)
+                tmem_st_16x256b_x4(tw, r);
                 kq_compute_quarter<FMT, 1>(tr, scr, lane, r);
-                if (more) kq_refill<FMT, 1>(nx, lane, tr);
-                KYB_KQ_PUBLISH()
-                KYB_KQ_STORE()
+                if (more) kq_refill<FMT, 1>(wk.ptr, lane, tr);
+                tmem_st_16x256b_x4(tw + 32u, r);
+                KYB_KQ_PUBLISH(0)
                 kq_compute_quarter<FMT, 2>(tr, scr, lane, r);
-                if (more) kq_refill<FMT, 2>(nx, lane, tr);
-                KYB_KQ_PUBLISH()
-                KYB_KQ_STORE()
+                if (more) kq_refill<FMT, 2>(wk.ptr, lane, tr);
+                KYB_KQ_WAIT(1)
+                tmem_st_16x256b_x4(tw + 64u, r);
                 kq_compute_quarter<FMT, 3>(tr, scr, lane, r);
-                if (more) kq_refill<FMT, 3>(nx, lane, tr);
-                KYB_KQ_PUBLISH()                                                     // its warp barrier also ends every lane's reads of this tile's scales
+                if (more) kq_refill<FMT, 3>(wk.ptr, lane, tr);
+                tmem_st_16x256b_x4(tw + 96u, r);
+                KYB_KQ_PUBLISH(1)                                                       // its warp barrier also ends every lane's reads of this tile's scales
                 if (more) {
-                    kq_prep_scales<FMT>(tr, scr, lane);                              // tr.sc holds the next tile's scale bytes
+                    kq_prep_scales<FMT>(tr, scr, lane);                                 // tr.sc holds the next tile's scale bytes
                     __syncwarp();
-                    if (more2) kq_refill_scales<FMT>(nx + TB, lane, tr);
+                    kq_compute_quarter<FMT, 0>(tr, scr, lane, r);                       // quarter 0 of the next tile
                 }
-                KYB_KQ_STORE()
                 if (more) {
-                    kq_compute_quarter<FMT, 0>(tr, scr, lane, r);                    // quarter 0 of the next tile
-                    if (more2) kq_refill<FMT, 0>(nx + TB, lane, tr);
+                    wk.advance(p, num_items, stride, rank, tord, kp, q, half);
+                    if (wk.ok) {
+                        kq_refill_scales<FMT>(wk.ptr, lane, tr);
+                        kq_refill<FMT, 0>(wk.ptr, lane, tr);
+                    }
                 }
-                KYB_KQ_PUBLISH()
+                parity ^= 1u;
             }
+#undef KYB_KQ_WAIT
 #undef KYB_KQ_PUBLISH
-#undef KYB_KQ_STORE
         }
     }
-    if (warp >= 2 && warp < 6 && lane == 0 && (p.tma_out || p.part)) tma_store_wait_all();   // the staging buffer must outlive its stores
+    if (warp == 2 && lane == 0 && p.tma_out) tma_store_wait_all();                      // the staging buffer must outlive its stores
     if (failed) atomicExch(p.status, KYB_DEV_TIMEOUT_GEMM);
     tc_fence_before();
-    __syncthreads();
+    if constexpr (PAIR) cluster_sync_all();                                            // neither CTA frees tensor memory or leaves while the other may still signal it
+    else __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, TMEM_COLS);
+        if constexpr (PAIR) tmem_dealloc_pair(tmem_base, TMEM_COLS);
+        else tmem_dealloc(tmem_base, TMEM_COLS);
     }
 }
-
 
 // split-k, second step: d [m, n] = sat(gscale * (part[0] + part[1] + ... in k order)), eight columns per thread
 __global__ void gemm_kq_reduce_kernel(const float* __restrict__ part, int ksplit, int m, int mpad, int n, int64_t ldp, float gscale, __half* __restrict__ d, int64_t ldd) {
@@ -889,325 +992,111 @@ __global__ void gemm_kq_reduce_kernel(const float* __restrict__ part, int ksplit
     }
 }
 
-// ------------------------------------------------------------------------------------------------ the dense form by CTA pairs (tcgen05 cta_group::2)
-// A pair of CTAs computes a 256 x 256 tile of D: each CTA holds 128 activation rows (TMA) and decodes ONE HALF of the 256 weight rows (8 row tiles) of a
-// 128-input stage; one MMA of the pair's leader runs on both tensor cores. Per SM and per flop the decode work, the decoder stores and the B operand reads are
-// half of those of a one-CTA item with two activation blocks, which is what bounds that form (shared-memory bandwidth). The 16 decoder warps of a CTA are
-// (row tile w & 7, quarter parity w >> 3): a warp decodes quarters hq and hq + 2 of every T16 tile of its row tile, one per stage (a stage is 128 inputs =
-// two 64-input K-halves; quarter hq or hq + 2 of the tile lands in K-half hq). Barriers as in the NVFP4 pair kernel: full[s] in the leader (the leader's
-// producer with the byte count of both CTAs' activation tiles + the 32 decoder warps of both CTAs, the peer's by remote arrive), empty[s] and acc_full in each
-// CTA (commit to the pair), acc_empty in the leader (8 epilogue warps). Two accumulators alternate. Every wait is bounded.
-// The decoder warps of the peer arrive on the leader's barrier with the plain (CTA-scope release) form of the remote arrive, as the vendor's own pipelines do
-// for remote arrivals: by then the warp's stores sit in its own CTA's shared memory behind a proxy fence, which is where the leader's MMA reads them. With
-// release at cluster scope on each of the 32 arrivals per stage the kernel ran at 950 TFLOP/s instead of 1430.
-constexpr uint32_t KP_A_BYTES = 2 * KQ_A_SUB, KP_B_BYTES = 2 * 128 * KQ_BK * 2, KP_STAGE_BYTES = KP_A_BYTES + KP_B_BYTES;   // 32 K + 32 K per 128-input stage
-constexpr int KP_STAGES = 3;
-
-// registers that only quarter P of the tile used are refilled from the next tile right after P has been computed (this warp uses two quarters of a tile)
-template <int FMT, int P>
-__device__ __forceinline__ void kq_refill_pair(const uint8_t* next, int lane, KqTile<FMT>& tr) {
-    if constexpr (FMT == KYB_FMT_Q4_K || FMT == KYB_FMT_NVFP4 || FMT == KYB_FMT_IQ4_XS) {
-        tr.q[P] = ldg128s(next + (P * 32 + lane) * 16);
-    } else if constexpr (FMT == KYB_FMT_Q2_K) {
-        tr.q[P >> 1] = ldg128s(next + ((P >> 1) * 32 + lane) * 16);
-    } else if constexpr (FMT == KYB_FMT_Q5_K) {
-        tr.q[P] = ldg128s(next + (P * 32 + lane) * 16);
-        const uint2 hb = ldg64s(next + 2048 + lane * 16 + ((P & 2) ? 8 : 0));
-        if constexpr ((P & 2) == 0) tr.q[4].x = hb.x, tr.q[4].y = hb.y;
-        else tr.q[4].z = hb.x, tr.q[4].w = hb.y;
-    } else if constexpr (FMT == KYB_FMT_Q8_0) {
-        tr.q[2 * P] = ldg128s(next + (2 * P * 32 + lane) * 16);
-        tr.q[2 * P + 1] = ldg128s(next + ((2 * P + 1) * 32 + lane) * 16);
-    } else if constexpr (FMT == KYB_FMT_Q6_K) {
-        tr.q[P] = ldg128s(next + (P * 32 + lane) * 16);
-        tr.q[4 + (P >> 1)] = ldg128s(next + 2048 + ((P >> 1) * 32 + lane) * 16);
-    } else {
-        tr.q[P >> 1] = ldg128s(next + ((P >> 1) * 32 + lane) * 16);
-        const uint2 hb = ldg64s(next + 1024 + lane * 16 + ((P & 2) ? 8 : 0));
-        if constexpr ((P & 2) == 0) tr.q[2].x = hb.x, tr.q[2].y = hb.y;
-        else tr.q[2].z = hb.x, tr.q[2].w = hb.y;
-    }
-}
-
-struct KpTile {
-    int m0, n0;      // this CTA's first activation row, first weight row of the 256-wide tile
-};
-__device__ __forceinline__ KpTile kp_tile(const KqParams& p, int t, uint32_t rank) {
-    KpTile it;
-    const int tn = t / p.tiles_m, tm = t - tn * p.tiles_m;                          // m fastest: the pairs running together share the weight rows
-    it.n0 = tn * KQ_BN, it.m0 = tm * 256 + (int)rank * 128;
-    return it;
-}
-
-template <int FMT, int HQ>
-__device__ __forceinline__ bool kp_decode(const KqParams& p, const int num_items, const int pair, const int pairs, const uint32_t rank, const int rt8, const int lane,
-                                          const uint32_t smem0, const uint32_t scr, const uint32_t full_leader0, const uint32_t empty0) {
-    constexpr int TB = kyb_tile_bytes(FMT);
-    const int g = lane >> 2, tq = lane & 3;
-    const uint32_t row_off = (uint32_t)(2 * rt8) * 1024u + (uint32_t)g * 128u + 8u * (uint32_t)(tq & 1);
-    const bool odd = (g & 1) != 0;
-    uint32_t cx[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) cx[i] = (uint32_t)(((2 * (i ^ (odd ? 2 : 0)) + (tq >> 1)) ^ g) * 16);
-    uint32_t parity = 1;
-    int s = 0;
-    bool failed = false;
-    for (int t = pair; t < num_items && !failed; t += pairs) {
-        const KpTile it = kp_tile(p, t, rank);
-        const int rt = min((it.n0 >> 4) + (int)rank * 8 + rt8, p.rt_total - 1);
-        const uint8_t* tp = p.t16 + (size_t)rt * (size_t)p.nb * TB;
-        KqTile<FMT> tr;
-        uint32_t r[16];
-        kq_load<FMT>(tp, lane, tr);
-        kq_prep_scales<FMT>(tr, scr, lane);
-        __syncwarp();
-        if (p.nb > 1) kq_refill_scales<FMT>(tp + TB, lane, tr);
-        kq_compute_quarter<FMT, HQ>(tr, scr, lane, r);
-        if (p.nb > 1) kq_refill_pair<FMT, HQ>(tp + TB, lane, tr);
-#define KYB_KP_STORE()                                                                                            \
-    {                                                                                                             \
-        if (!mbar_wait_fast(empty0 + 8 * s, parity)) failed = true;                                               \
-        const uint32_t b_dst = smem0 + s * KP_STAGE_BYTES + KP_A_BYTES + HQ * 16384u + row_off;                   \
-        kq_store_quarter(b_dst, b_dst + 1024u, cx, odd, r);                                                       \
-    }
-#define KYB_KP_PUBLISH()                                                                                          \
-    {                                                                                                             \
-        fence_proxy_async_smem();                                                                                 \
-        __syncwarp();                                                                                             \
-        if (lane == 0) mbar_arrive_remote(full_leader0 + 8 * s);                                                  \
-        if (++s == KP_STAGES) s = 0, parity ^= 1u;                                                                \
-    }
-        for (int kb = 0; kb < p.nb && !failed; ++kb) {
-            const bool more = kb + 1 < p.nb, more2 = kb + 2 < p.nb;
-            const uint8_t* nx = tp + (size_t)(kb + 1) * TB;
-            KYB_KP_STORE()                                                       // quarter HQ: inputs [0, 128) of the tile
-            kq_compute_quarter<FMT, HQ + 2>(tr, scr, lane, r);
-            if (more) kq_refill_pair<FMT, HQ + 2>(nx, lane, tr);
-            KYB_KP_PUBLISH()                                                     // its warp barrier also ends every lane's reads of this tile's scales
-            if (more) {
-                kq_prep_scales<FMT>(tr, scr, lane);                              // tr.sc holds the next tile's scale bytes
-                __syncwarp();
-                if (more2) kq_refill_scales<FMT>(nx + TB, lane, tr);
-            }
-            KYB_KP_STORE()                                                       // quarter HQ + 2: inputs [128, 256)
-            if (more) {
-                kq_compute_quarter<FMT, HQ>(tr, scr, lane, r);
-                if (more2) kq_refill_pair<FMT, HQ>(nx + TB, lane, tr);
-            }
-            KYB_KP_PUBLISH()
-        }
-#undef KYB_KP_STORE
-#undef KYB_KP_PUBLISH
-    }
-    return failed;
-}
-
-template <int FMT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(KQ_THREADS, 1)
-    gemm_kq_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ KqOutMaps outs, const KqParams p, const int num_items) {
-    extern __shared__ __align__(1024) uint8_t smem_raw[];
-    const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t scr0 = smem0 + (uint32_t)KP_STAGES * KP_STAGE_BYTES;
-    const uint32_t stg0 = scr0 + KQ_DW * KQ_SCR;                                    // epilogue staging, 4 warps
-    const uint32_t bars = stg0 + 4 * KQ_STG;                                        // full[STAGES], empty[STAGES], acc_full[2], acc_empty[2], tmem slot
-    const uint32_t full0 = bars, empty0 = bars + 8 * KP_STAGES, accf0 = bars + 16 * KP_STAGES, acce0 = accf0 + 16, tmem_slot = acce0 + 16;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rank = cluster_rank();
-    const int pair = (int)(blockIdx.x >> 1), pairs = (int)(gridDim.x >> 1);
-    const int kstages = p.k / 128;
-    constexpr uint32_t TMEM_COLS = 512;
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < KP_STAGES; ++s) mbar_init_a(full0 + 8 * s, 2 * KQ_DW + 1), mbar_init_a(empty0 + 8 * s, 1);
-        for (int a = 0; a < 2; ++a) mbar_init_a(accf0 + 8 * a, 1), mbar_init_a(acce0 + 8 * a, 8);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        prefetch_tmap(&tma_a);
-    }
-    if (warp == 1) tmem_alloc_pair(tmem_slot, TMEM_COLS);
-    tc_fence_before();
-    cluster_sync_all();                                                            // both CTAs' barriers exist before either signals the other
-    tc_fence_after();
-    const uint32_t tmem_base = lds32(tmem_slot);
-    const uint32_t full_leader0 = map_to_rank(full0, 0);
-    bool failed = false;
-
-    if (warp == 0) {
-        // ---- TMA producer: this CTA's 128 activation rows, two 64-input boxes per stage
-        if (elect_one()) {
-            uint32_t parity = 1;
-            int s = 0;
-            for (int t = pair; t < num_items && !failed; t += pairs) {
-                const KpTile it = kp_tile(p, t, rank);
-                for (int ks = 0; ks < kstages && !failed; ++ks) {
-                    if (!mbar_wait_fast(empty0 + 8 * s, parity)) failed = true;
-                    const uint32_t a_dst = smem0 + s * KP_STAGE_BYTES;
-                    if (rank == 0) mbar_expect_tx_a(full0 + 8 * s, 2 * KP_A_BYTES);
-                    tma_load_2d_pair(a_dst, &tma_a, ks * 128, it.m0, full_leader0 + 8 * s);
-                    tma_load_2d_pair(a_dst + KQ_A_SUB, &tma_a, ks * 128 + 64, it.m0, full_leader0 + 8 * s);
-                    if (++s == KP_STAGES) s = 0, parity ^= 1u;
-                }
-            }
-        }
-    } else if (warp == 1) {
-        // ---- MMA issuer: the pair's leader
-        if (rank == 0 && elect_one()) {
-            constexpr uint32_t idesc = umma_idesc_f16(256, KQ_BN);
-            uint32_t parity = 0;
-            int s = 0;
-            uint32_t cnt = 0;
-            for (int t = pair; t < num_items && !failed; t += pairs, ++cnt) {
-                const uint32_t slot = cnt & 1u;
-                if (!mbar_wait_fast(acce0 + 8 * slot, ((cnt >> 1) & 1u) ^ 1u)) failed = true;           // both CTAs' epilogues have drained the slot
-                tc_fence_after();
-                const uint32_t tmem_d = tmem_base + slot * KQ_BN;
-                for (int ks = 0; ks < kstages && !failed; ++ks) {
-                    if (!mbar_wait_fast(full0 + 8 * s, parity)) failed = true;
-                    tc_fence_after();
-                    const uint32_t a_src = smem0 + s * KP_STAGE_BYTES, b_src = a_src + KP_A_BYTES;
-#pragma unroll
-                    for (int kh = 0; kh < 2; ++kh) {
-                        const uint64_t adesc = umma_desc_sw128(a_src + kh * KQ_A_SUB), bdesc = umma_desc_sw128(b_src + kh * 16384u);
-#pragma unroll
-                        for (int kk = 0; kk < KQ_BK / 16; ++kk) umma_f16_pair(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (ks | kh | kk) != 0);
-                    }
-                    umma_commit_pair(empty0 + 8 * s);
-                    if (++s == KP_STAGES) s = 0, parity ^= 1u;
-                }
-                umma_commit_pair(accf0 + 8 * slot);
-            }
-        }
-    } else if (warp < 6) {
-        // ---- epilogue: this CTA's 128 rows x 256 columns, staged tiled bulk stores
-        const int q = warp & 3;
-        const uint32_t acce_leader0 = map_to_rank(acce0, 0);
-        uint32_t cnt = 0;
-        for (int t = pair; t < num_items; t += pairs, ++cnt) {
-            const KpTile it = kp_tile(p, t, rank);
-            const uint32_t slot = cnt & 1u;
-            if (!mbar_wait_fast(accf0 + 8 * slot, (cnt >> 1) & 1u)) failed = true;
-            tc_fence_after();
-            const uint32_t stg = stg0 + (uint32_t)q * KQ_STG;
-            const int row0 = it.m0 + q * 32;
-#pragma unroll 1
-            for (int c = 0; c < KQ_BN; c += 32) {
-                uint32_t v[32];
-                tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + slot * KQ_BN + (uint32_t)c, v);
-                tmem_ld_wait();
-                uint32_t w[16];
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    __half2 h = sat_half2(__uint_as_float(v[2 * j]) * p.gscale, __uint_as_float(v[2 * j + 1]) * p.gscale);
-                    w[j] = *reinterpret_cast<uint32_t*>(&h);
-                }
-                epilogue_stage_store(outs, 1, stg, lane, w, it.n0 + c, row0, !failed && row0 < p.m && it.n0 + c < p.n);
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(acce_leader0 + 8 * slot);
-        }
-    } else {
-        // ---- decoders
-        const int dw = warp - 6;
-        const uint32_t scr = scr0 + dw * KQ_SCR;
-        if (dw < 8) failed = kp_decode<FMT, 0>(p, num_items, pair, pairs, rank, dw, lane, smem0, scr, full_leader0, empty0);
-        else failed = kp_decode<FMT, 1>(p, num_items, pair, pairs, rank, dw - 8, lane, smem0, scr, full_leader0, empty0);
-    }
-    if (warp >= 2 && warp < 6 && lane == 0) tma_store_wait_all();                      // the staging buffer must outlive its stores
-    if (failed) atomicExch(p.status, KYB_DEV_TIMEOUT_GEMM);
-    tc_fence_before();
-    cluster_sync_all();                                                            // neither CTA frees tensor memory or leaves while the other may still signal it
-    if (warp == 1) {
-        tc_fence_after();
-        tmem_dealloc_pair(tmem_base, TMEM_COLS);
-    }
-}
-
 }  // namespace kyb
 
 namespace {
 
-int kq_launch(int fmt, const CUtensorMap& ta, const KybOutMaps& outs, kyb::KqParams p, int num_items, cudaStream_t st) {
-    static std::mutex mu;
-    static unsigned done[KYB_FMT_COUNT] = {};
-    static int sms = 0;
-    int dev = 0;
-    KYB_CUDA(cudaGetDevice(&dev));
-    const void* kern = fmt == KYB_FMT_Q4_K   ? (const void*)kyb::gemm_kq_kernel<KYB_FMT_Q4_K>
-                       : fmt == KYB_FMT_Q6_K ? (const void*)kyb::gemm_kq_kernel<KYB_FMT_Q6_K>
-                       : fmt == KYB_FMT_Q3_K ? (const void*)kyb::gemm_kq_kernel<KYB_FMT_Q3_K>
-                       : fmt == KYB_FMT_Q5_K ? (const void*)kyb::gemm_kq_kernel<KYB_FMT_Q5_K>
-                       : fmt == KYB_FMT_Q8_0 ? (const void*)kyb::gemm_kq_kernel<KYB_FMT_Q8_0>
-                       : fmt == KYB_FMT_Q2_K ? (const void*)kyb::gemm_kq_kernel<KYB_FMT_Q2_K>
-                       : fmt == KYB_FMT_IQ4_XS ? (const void*)kyb::gemm_kq_kernel<KYB_FMT_IQ4_XS>
-                                             : (const void*)kyb::gemm_kq_kernel<KYB_FMT_NVFP4>;
-    const uint32_t stage_bytes = (uint32_t)p.msub * kyb::KQ_A_SUB + kyb::KQ_B_BYTES;
-    const size_t fixed = (size_t)kyb::KQ_DW * kyb::KQ_SCR + 4 * (p.wide ? 2 : 1) * kyb::KQ_STG + 1024 + 256 + (p.tb ? 2 * kyb::KQ_TORD : 0);
-    const size_t cap = 227 * 1024;
-    p.stages = (int)std::min<size_t>(8, (cap - fixed) / stage_bytes);
-    const size_t smem = (size_t)p.stages * stage_bytes + fixed;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        if (!(done[fmt] & (1u << (dev & 31)))) {
-            KYB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
-            done[fmt] |= 1u << (dev & 31);
-        }
-        if (!sms) KYB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+template <bool PAIR>
+const void* kq_kernel_ptr(int fmt) {
+    switch (fmt) {
+        case KYB_FMT_Q4_K: return (const void*)kyb::gemm_kq_kernel<KYB_FMT_Q4_K, PAIR>;
+        case KYB_FMT_Q6_K: return (const void*)kyb::gemm_kq_kernel<KYB_FMT_Q6_K, PAIR>;
+        case KYB_FMT_Q3_K: return (const void*)kyb::gemm_kq_kernel<KYB_FMT_Q3_K, PAIR>;
+        case KYB_FMT_Q5_K: return (const void*)kyb::gemm_kq_kernel<KYB_FMT_Q5_K, PAIR>;
+        case KYB_FMT_Q8_0: return (const void*)kyb::gemm_kq_kernel<KYB_FMT_Q8_0, PAIR>;
+        case KYB_FMT_Q2_K: return (const void*)kyb::gemm_kq_kernel<KYB_FMT_Q2_K, PAIR>;
+        case KYB_FMT_IQ4_XS: return (const void*)kyb::gemm_kq_kernel<KYB_FMT_IQ4_XS, PAIR>;
+        default: return (const void*)kyb::gemm_kq_kernel<KYB_FMT_NVFP4, PAIR>;
     }
-    void* args[] = {(void*)&ta, (void*)&outs, (void*)&p, (void*)&num_items};
-    KYB_CUDA(cudaLaunchKernel(kern, dim3((unsigned)std::min(num_items, sms)), dim3(kyb::KQ_THREADS), args, smem, st));
-    return kyb_launch_check("gemm_kq");
 }
 
-// the dense form by CTA pairs; KYB_EUNSUPPORTED when the device cannot hold a pair of these CTAs at once or the tile count suits the one-CTA kernel better (the
-// caller then takes that kernel)
-int kq_launch_pair(int fmt, const CUtensorMap& ta, const KybOutMaps& outs, kyb::KqParams p, cudaStream_t st) {
+constexpr size_t KQ_SMEM_CAP = 227 * 1024;
+constexpr size_t KQ_RING = 128 * 1024;                  // activation ring
+constexpr size_t KQ_SMEM_FIXED = 1024 + 2 * kyb::KQ_STG + (size_t)kyb::KQ_DW * kyb::KQ_SCR + 112 + 2 * kyb::KQ_TORD;
+
+int kq_sms() {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0, v = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
+        (void)cudaGetLastError();
+        sms = v;
+    }
+    return sms;
+}
+
+// shared-memory attribute once per device, format and form; by pairs also how many CTA pairs the device holds at once (0: none, take the one-CTA form)
+template <bool PAIR>
+int kq_configure(int fmt, int* pairs) {
     static std::mutex mu;
     static unsigned done[KYB_FMT_COUNT] = {};
     static int pairs_max[KYB_FMT_COUNT][32] = {};
     int dev = 0;
     KYB_CUDA(cudaGetDevice(&dev));
-    const void* kern = fmt == KYB_FMT_Q4_K   ? (const void*)kyb::gemm_kq_pair_kernel<KYB_FMT_Q4_K>
-                       : fmt == KYB_FMT_Q6_K ? (const void*)kyb::gemm_kq_pair_kernel<KYB_FMT_Q6_K>
-                       : fmt == KYB_FMT_Q3_K ? (const void*)kyb::gemm_kq_pair_kernel<KYB_FMT_Q3_K>
-                       : fmt == KYB_FMT_Q5_K ? (const void*)kyb::gemm_kq_pair_kernel<KYB_FMT_Q5_K>
-                       : fmt == KYB_FMT_Q8_0 ? (const void*)kyb::gemm_kq_pair_kernel<KYB_FMT_Q8_0>
-                       : fmt == KYB_FMT_Q2_K ? (const void*)kyb::gemm_kq_pair_kernel<KYB_FMT_Q2_K>
-                       : fmt == KYB_FMT_IQ4_XS ? (const void*)kyb::gemm_kq_pair_kernel<KYB_FMT_IQ4_XS>
-                                             : (const void*)kyb::gemm_kq_pair_kernel<KYB_FMT_NVFP4>;
-    constexpr size_t smem = (size_t)kyb::KP_STAGES * kyb::KP_STAGE_BYTES + (size_t)kyb::KQ_DW * kyb::KQ_SCR + 4 * kyb::KQ_STG + 1024 + 256;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        if (!(done[fmt] & (1u << (dev & 31)))) {
-            KYB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const void* kern = kq_kernel_ptr<PAIR>(fmt);
+    std::lock_guard<std::mutex> lk(mu);
+    if (!(done[fmt] & (1u << (dev & 31)))) {
+        KYB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KQ_SMEM_CAP));
+        if (PAIR) {
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
             cudaLaunchConfig_t qc = {};
-            qc.gridDim = dim3(2), qc.blockDim = dim3(kyb::KQ_THREADS), qc.dynamicSmemBytes = smem;
+            qc.gridDim = dim3(2), qc.blockDim = dim3(kyb::KQ_THREADS), qc.dynamicSmemBytes = KQ_SMEM_FIXED + KQ_RING, qc.attrs = attr, qc.numAttrs = 1;
             int nc = 0;
             if (cudaOccupancyMaxActiveClusters(&nc, kern, &qc) != cudaSuccess || nc <= 0) {
                 (void)cudaGetLastError();
                 nc = 0;
             }
             pairs_max[fmt][dev & 31] = nc;
-            done[fmt] |= 1u << (dev & 31);
         }
+        done[fmt] |= 1u << (dev & 31);
     }
-    const int pm = pairs_max[fmt][dev & 31];
-    if (pm <= 0) return KYB_EUNSUPPORTED;
-    p.msub = 2;
-    p.tiles_m = (p.m + 255) / 256;
-    const int num_items = p.tiles_n * p.tiles_m;
-    // more tiles than pairs but no more than SMs: the one-CTA kernel runs them all at once, pairs would need a second, poorly filled wave (12288 -> 3072 at
-    // M = 2048: 96 tiles, 156 us against 170 us)
-    if (num_items > pm && num_items <= 2 * pm) return KYB_EUNSUPPORTED;
-    const int pairs = std::min(num_items, pm);
+    if (pairs) *pairs = pairs_max[fmt][dev & 31];
+    return KYB_OK;
+}
+
+// units: CTAs (one-CTA form) or pairs that may run at once
+template <bool PAIR>
+int kq_launch(int fmt, const CUtensorMap& ta, const KybOutMaps& outs, kyb::KqParams p, int num_items, int units, cudaStream_t st) {
+    if (int rc = kq_configure<PAIR>(fmt, nullptr)) return rc;
+    // a stage of the activation ring is 128 inputs of up to 128 rows per CTA (the one-CTA form with wider items: 256)
+    p.bstages = !PAIR && p.mt > 128 ? 2 : 4;
+    p.bstage_bytes = (uint32_t)(KQ_RING / p.bstages);
+    const size_t smem = KQ_SMEM_FIXED + KQ_RING;
+    const int n = std::min(num_items, units);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(PAIR ? 2 * n : n)), cfg.blockDim = dim3(kyb::KQ_THREADS), cfg.dynamicSmemBytes = smem, cfg.stream = st, cfg.attrs = attr, cfg.numAttrs = PAIR ? 1 : 0;
     void* args[] = {(void*)&ta, (void*)&outs, (void*)&p, (void*)&num_items};
-    KYB_CUDA(cudaLaunchKernel(kern, dim3((unsigned)(2 * pairs)), dim3(kyb::KQ_THREADS), args, smem, st));
-    return kyb_launch_check("gemm_kq_pair");
+    KYB_CUDA(cudaLaunchKernelExC(&cfg, kq_kernel_ptr<PAIR>(fmt), args));
+    return kyb_launch_check("gemm_kq");
+}
+
+// Activation rows per item (a multiple of 32, at most 256) for `tiles_n` column tiles on `units` CTAs or pairs: the whole rounds of equal items that cost least. A
+// stage of an item costs its MMAs (2 clocks per row) but never less than the decode of its weights (`dec` clocks), an item about 12 stages' worth of start and end.
+int kq_rows_per_item(int64_t m, int64_t tiles_n, int units, double stages, double dec, double* cost_out) {
+    int best = 0;
+    double best_cost = 0.0;
+    for (int tm = (int)((m + 255) / 256), last = 0; tm <= (int)((m + 31) / 32) && tm <= 4096; ++tm) {
+        const int mt = (int)((m + (int64_t)tm * 32 - 1) / ((int64_t)tm * 32)) * 32;
+        if (mt == last) continue;
+        last = mt;
+        if (mt < 96 && best) break;                                                    // narrower items are bound by the decode: more of them never pays
+        const int64_t items = tiles_n * ((m + mt - 1) / mt), rounds = (items + units - 1) / units;
+        const double cost = (double)rounds * (stages * std::max(dec, 2.0 * mt) + 4000.0);
+        if (!best || cost < 0.97 * best_cost) best = mt, best_cost = cost;
+    }
+    if (cost_out) *cost_out = best_cost;
+    return best;
 }
 
 }  // namespace
 
 static int kq_dense(int fmt, const void* t16, int64_t n, int64_t k, const void* a, int64_t lda, int64_t m, float gscale, void* const* d, int nout, int64_t ldd,
-                    int64_t col0, int msub, void* stream, bool pair_ok = true, int ksplit = 1, float* part = nullptr) {
+                    int64_t col0, int msub, void* stream, int ksplit = 1, float* part = nullptr) {
     KYB_REQUIRE(fmt >= 0 && fmt < KYB_FMT_COUNT, "unknown weight format %d", fmt);
     KYB_REQUIRE(t16 && a, "null pointer");
     KYB_REQUIRE(m > 0 && n > 0 && k > 0 && k % 256 == 0, "m=%lld n=%lld k=%lld: k must be a positive multiple of 256", (long long)m, (long long)n, (long long)k);
@@ -1215,64 +1104,54 @@ static int kq_dense(int fmt, const void* t16, int64_t n, int64_t k, const void* 
     KYB_REQUIRE(((uintptr_t)a & 15) == 0 && ((uintptr_t)t16 & 15) == 0, "a and t16 must be 16-byte aligned");
     KYB_REQUIRE(m < (1ll << 31) && n < (1ll << 31) && k < (1ll << 24), "dimension too large");
     KYB_REQUIRE(msub >= 0 && msub <= 2, "msub is 0 (automatic), 1 or 2");
-    const bool automatic = msub == 0;                                              // a given msub asks for the one-CTA kernel with that many activation blocks per item
     unsigned int* status = kyb_device_status_word();
     KYB_REQUIRE(status, "could not set up the device status word");
-    CUtensorMap ta;
-    if (int rc = kyb_make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a, (uint64_t)m, (uint64_t)k, (uint64_t)lda * 2, 128, kyb::KQ_BK)) return rc;
     kyb::KqParams p;
+    memset(&p, 0, sizeof(p));
     p.t16 = (const uint8_t*)t16, p.ldd = ldd, p.m = (int)m, p.n = (int)n, p.k = (int)k, p.nb = (int)(k / 256), p.rt_total = (int)((n + 15) / 16);
-    p.nout = nout;
-    for (int i = 0; i < 8; ++i) p.d[i] = i < nout ? (__half*)d[i] + col0 : nullptr;
-    p.gscale = gscale, p.status = status, p.tb = nullptr, p.off = nullptr, p.row_map = nullptr, p.gs = nullptr, p.experts = 0;
-    p.tiles_n = (int)((n + kyb::KQ_BN - 1) / kyb::KQ_BN);
-    p.ksplit = ksplit, p.mpad = 0, p.part = ksplit > 1 ? part : nullptr, p.ldp = (int64_t)p.tiles_n * kyb::KQ_BN;
-    if (!msub) {
-        // two activation blocks per item halve the decode work per flop, but they halve the number of items and keep both accumulators busy (no overlap of
-        // the epilogue with the next item): one block when the rows fit one block, when two-block items would leave more than half of the SMs idle, or when the
-        // epilogue also feeds other GPUs (its peer stores then overlap the next item's MMAs)
-        int dev = 0, sms = 148;
-        if (cudaGetDevice(&dev) == cudaSuccess) (void)cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const int64_t items2 = (int64_t)p.tiles_n * ((m + 255) / 256);
-        msub = (m <= 128 || items2 * 2 < sms || nout > 1) ? 1 : 2;
+    p.nout = nout, p.gscale = gscale, p.status = status;
+    for (int i = 0; i < nout; ++i) p.d[i] = (__half*)d[i] + col0;
+    p.ksplit = ksplit, p.mpad = (int)m, p.part = ksplit > 1 ? part : nullptr, p.ldp = (n + 255) / 256 * 256;
+    // a given msub asks for the one-CTA form with that many 128-row blocks per item
+    int pairs = 0;
+    const int sms = kq_sms();
+    if (msub == 0)
+        if (int rc = kq_configure<true>(fmt, &pairs)) return rc;
+    const double stages = 4.0 * p.nb / ksplit;
+    bool pair = false;
+    if (msub) {
+        p.mt = 128 * msub;
+    } else {
+        double c1 = 0.0, c2 = 0.0;
+        const int mt1 = kq_rows_per_item(m, (n + 127) / 128 * ksplit, sms, stages, 300.0, &c1);
+        const int mt2 = pairs > 0 ? kq_rows_per_item(m, (n + 255) / 256 * ksplit, pairs, stages, 300.0, &c2) : 0;
+        pair = pairs > 0 && c2 <= 1.02 * c1;
+        p.mt = pair ? mt2 : mt1;
     }
-    p.msub = msub;
-    p.tiles_m = (int)((m + 128 * p.msub - 1) / (128 * p.msub));
-    // tiled bulk stores need 16-byte aligned bases and row pitches; otherwise the epilogue stores from registers
+    CUtensorMap ta;                                                                 // one box is 64 inputs of all the rows that a CTA loads for an item
+    p.box_rows = (uint32_t)(pair ? p.mt / 2 : p.mt);
+    if (int rc = kyb_make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a, (uint64_t)m, (uint64_t)k, (uint64_t)lda * 2, p.box_rows, 64)) return rc;
+    p.tiles_n = (int)(pair ? (n + 255) / 256 : (n + 127) / 128);
+    p.tiles_m = (int)((m + p.mt - 1) / p.mt);
+    // tiled bulk stores need 16-byte aligned bases and row pitches; otherwise the epilogue stores row pieces
     KybOutMaps outs;
     memset(&outs, 0, sizeof(outs));
     p.col0 = (int)col0;
-    p.tma_out = (ldd % 8 == 0 && col0 % 8 == 0) ? 1 : 0;
+    p.tma_out = (ldd % 8 == 0 && col0 % 8 == 0 && ksplit == 1) ? 1 : 0;
     for (int i = 0; i < nout && p.tma_out; ++i)
         if ((uintptr_t)d[i] & 15) p.tma_out = 0;
-    p.wide = (p.tma_out && nout > 1) ? 1 : 0;
-    p.t16b = nullptr, p.gsb = nullptr, p.glu = 0, p.limit = 0.f;
     for (int i = 0; i < nout && p.tma_out; ++i)
-        if (int rc = kyb_make_tmap_2d(&outs.m[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, d[i], (uint64_t)m, (uint64_t)(col0 + n), (uint64_t)ldd * 2, 32, p.wide ? 64 : 32,
-                                      p.wide ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B))
-            return rc;
-    if (ksplit > 1) {
-        // split-k: the one-CTA kernel over (tile, k-range) items, whose staged stores go to the fp32 ranges (tensor map over part as 16-bit pairs), then the
-        // ranges are added
-        p.mpad = p.tiles_m * 128 * p.msub, p.tma_out = 0, p.wide = 0;
-        memset(&outs, 0, sizeof(outs));
-        if (int rc = kyb_make_tmap_2d(&outs.m[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, part, (uint64_t)ksplit * (uint64_t)p.mpad, (uint64_t)(2 * p.ldp), (uint64_t)p.ldp * 4, 32, 32,
-                                      CU_TENSOR_MAP_SWIZZLE_64B))
-            return rc;
-        if (int rc = kq_launch(fmt, ta, outs, p, p.tiles_n * p.tiles_m * ksplit, (cudaStream_t)stream)) return rc;
-        const int64_t threads = m * ((n + 7) / 8);
-        kyb::gemm_kq_reduce_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(part, ksplit, (int)m, p.mpad, (int)n, p.ldp, gscale, (__half*)d[0], ldd);
-        return kyb_launch_check("gemm_kq_reduce");
-    }
-    if (nout == 1 && p.tma_out && m > 128 && pair_ok && automatic) {
-        // one destination and at least two row blocks: CTA pairs (cta_group::2), each CTA decoding half of the 256 weight rows of a tile
-        if (int rc = kq_launch_pair(fmt, ta, outs, p, (cudaStream_t)stream); rc != KYB_EUNSUPPORTED) return rc;
-    }
-    return kq_launch(fmt, ta, outs, p, p.tiles_n * p.tiles_m, (cudaStream_t)stream);
+        if (int rc = kyb_make_tmap_2d(&outs.m[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, d[i], (uint64_t)m, (uint64_t)(col0 + n), (uint64_t)ldd * 2, 32, 64)) return rc;
+    const int items = p.tiles_n * p.tiles_m * ksplit;
+    if (int rc = pair ? kq_launch<true>(fmt, ta, outs, p, items, pairs, (cudaStream_t)stream) : kq_launch<false>(fmt, ta, outs, p, items, sms, (cudaStream_t)stream)) return rc;
+    if (ksplit == 1) return KYB_OK;
+    const int64_t threads = m * ((n + 7) / 8);
+    kyb::gemm_kq_reduce_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(part, ksplit, (int)m, p.mpad, (int)n, p.ldp, gscale, (__half*)d[0], ldd);
+    return kyb_launch_check("gemm_kq_reduce");
 }
 
 // D fp16 [m, n] (row stride ldd) = sat(gscale * A fp16 [m, k] (row stride lda) x W^T), W = T16 tiles of an [n, k] matrix of format fmt. msub = 0: the library
-// chooses (CTA pairs for more than 128 rows, else the one-CTA kernel); 1 or 2: the one-CTA kernel with that many blocks of 128 activation rows per work item.
+// chooses (CTA pairs, or the one-CTA form where that fills the SMs better); 1 or 2: the one-CTA form with up to that many blocks of 128 activation rows per item.
 // All forms give the same bits.
 extern "C" int kyb_gemm_kq(int fmt, const void* t16, int64_t n, int64_t k, const void* a, int64_t lda, int64_t m, float gscale, void* d, int64_t ldd, int msub,
                            void* stream) {
@@ -1324,7 +1203,7 @@ extern "C" int kyb_gemm_kq_splitk(int fmt, const void* t16, int64_t n, int64_t k
         return KYB_EWORKSPACE;
     }
     void* outs[1] = {d};
-    return kq_dense(fmt, t16, n, k, a, lda, m, gscale, outs, 1, ldd, 0, m > 128 ? 2 : 1, stream, false, split, (float*)workspace);
+    return kq_dense(fmt, t16, n, k, a, lda, m, gscale, outs, 1, ldd, 0, 0, stream, split, (float*)workspace);
 }
 
 // The same product with the all-gather of an N-sharded linear folded into the epilogue: every tile goes to the output matrix of every rank, at column col0.
@@ -1365,21 +1244,24 @@ static int kq_grouped(int fmt, const void* t16, const void* t16b, int64_t n, int
     unsigned int* status = kyb_device_status_word();
     KYB_REQUIRE(status, "could not set up the device status word");
     CUtensorMap ta;
-    if (int rc = kyb_make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a, (uint64_t)s, (uint64_t)k, (uint64_t)lda * 2, 128, kyb::KQ_BK)) return rc;
+    if (int rc = kyb_make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a, (uint64_t)s, (uint64_t)k, (uint64_t)lda * 2, 64, 64)) return rc;
     kyb::KqParams p;
+    memset(&p, 0, sizeof(p));
     p.t16 = (const uint8_t*)t16, p.ldd = ldd, p.m = (int)s, p.n = (int)n, p.k = (int)k, p.nb = (int)(k / 256);
-    p.nout = 1;
-    for (int i = 0; i < 8; ++i) p.d[i] = i == 0 ? (__half*)d : nullptr;
+    p.nout = 1, p.d[0] = (__half*)d;
     p.rt_total = (int)((int64_t)experts * n / 16);
     p.gscale = 1.0f, p.status = status, p.tb = (const uint32_t*)tb, p.off = (const uint32_t*)off, p.row_map = (const uint32_t*)row_map, p.gs = (const float*)gs, p.experts = experts;
-    p.msub = mt / 128;
-    p.ksplit = 1, p.mpad = 0, p.part = nullptr, p.ldp = 0;
+    p.mt = mt, p.ksplit = 1;
     p.t16b = (const uint8_t*)t16b, p.gsb = (const float*)gsb, p.glu = glu ? 1 : 0, p.limit = limit;
-    p.tiles_n = (int)(n / (glu ? kyb::KQ_BN / 2 : kyb::KQ_BN)), p.tiles_m = (int)((s + mt - 1) / mt) + experts;
-    p.tma_out = 0, p.col0 = 0, p.wide = 0;                                         // rows are scattered (row_map) or end inside a tile: no tensor map fits
+    int pairs = 0;
+    if (int rc = kq_configure<true>(fmt, &pairs)) return rc;
+    p.box_rows = 64;                                                               // segments have any number of rows: boxes of 64 as needed
+    p.tiles_n = (int)(n / (glu ? kyb::KQ_BN / 2 : kyb::KQ_BN)) / (pairs > 0 ? 2 : 1), p.tiles_m = (int)((s + mt - 1) / mt) + experts;
+    p.vec_out = (ldd % 8 == 0 && ((uintptr_t)d & 15) == 0) ? 1 : 0;                // rows are scattered (row_map) or end inside a tile: no tensor map fits
     KybOutMaps outs;
     memset(&outs, 0, sizeof(outs));
-    if (int rc = kq_launch(fmt, ta, outs, p, p.tiles_n * p.tiles_m, (cudaStream_t)stream)) return rc;
+    const int items = p.tiles_n * p.tiles_m;
+    if (int rc = pairs > 0 ? kq_launch<true>(fmt, ta, outs, p, items, pairs, (cudaStream_t)stream) : kq_launch<false>(fmt, ta, outs, p, items, kq_sms(), (cudaStream_t)stream)) return rc;
     return kyb_zero_tail_rows(d, ldd, n, row_map, (const uint32_t*)off + experts, s, (cudaStream_t)stream);   // slots that belong to no expert: rows of zeros
 }
 
