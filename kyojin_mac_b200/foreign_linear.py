@@ -3,6 +3,8 @@
 tensors, kernels are the sm_100a kernels behind include/kyb.h. There is no CPU path."""
 from __future__ import annotations
 
+import math
+
 import numpy as np
 import torch
 
@@ -245,7 +247,8 @@ class ForeignLinear(torch.nn.Module):
         shape = x.shape
         if shape[-1] != self.in_features:
             raise ValueError(f"input width {shape[-1]} != in_features {self.in_features}")
-        x2 = x.reshape(-1, shape[-1])
+        flat = x.dim() == 2                                                   # a decode step's call: two reshapes that change nothing cost 2 us
+        x2 = x if flat else x.reshape(-1, shape[-1])
         if x2.dtype != torch.float16:
             x2 = x2.to(torch.float16)
         if self._in_perm is not None and not permuted:
@@ -255,7 +258,7 @@ class ForeignLinear(torch.nn.Module):
             y = y.to(self.out_dtype)
         if self._bias is not None:
             y = y + self._bias
-        return y.reshape(*shape[:-1], self.out_features)
+        return y if flat else y.reshape(*shape[:-1], self.out_features)
 
 
 class SplitLinear(torch.nn.Module):
@@ -322,7 +325,7 @@ class ForeignSwitchGLU(torch.nn.Module):
     def forward(self, x, inds):
         lead, H = x.shape[:-1], x.shape[-1]
         K = inds.shape[-1]
-        T = int(np.prod(lead)) if len(lead) else 1
+        T = math.prod(lead)
         x2 = x.reshape(T, H).to(torch.float16)
         e32 = inds.reshape(-1).to(torch.int32)
         S = T * K
@@ -501,7 +504,7 @@ def _glu_call(self, x):
     (kyojin_mlx/foreign_linear.py:1882-1907). Any other case runs the module's own forward."""
     dn, g, u = self.down_proj, self.gate_proj, self.up_proj
     lead, H = x.shape[:-1], x.shape[-1]
-    R = int(np.prod(lead)) if len(lead) else 1
+    R = math.prod(lead)
     K = dn.in_features
     if dn.dev is None or R == 0 or R > F.GEMV_ROWS:
         return self._stock_call(x)

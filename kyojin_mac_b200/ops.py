@@ -8,8 +8,14 @@ from . import _lib, flags as F
 from .layout import FMT_ID, padded_rows
 
 
+# The current stream's handle without a torch.cuda.Stream object around it: every launch asks for it (3.2 us through torch.cuda.current_stream(), 0.2 us so).
+_raw_stream, _cur_device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    if _raw_stream is None or not torch.cuda.is_initialized():
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_cur_device())
 
 
 def _fmt(fmt) -> int:
@@ -96,17 +102,19 @@ def gemv(fmt, t16: torch.Tensor, n: int, k: int, x: torch.Tensor, gscale: float 
             raise ValueError("the gated form takes two float16 tensors of one shape")
         if x2.stride() != x.stride():
             x, x2 = x.contiguous(), x2.contiguous()
-    m = x.shape[0]
-    y = out if out is not None else torch.empty((m, n), dtype=torch.float16, device=x.device)
+    m, fid = x.shape[0], _fmt(fmt)
+    y = out if out is not None else x.new_empty((m, n))
     L = _lib.lib()
-    need = L.kyb_gemv_workspace_bytes(_fmt(fmt), n, k, m)
+    need = L.kyb_gemv_workspace_bytes(fid, n, k, m)
     ws = workspace(x.device, need) if need else None
     wp, wn = (ws.data_ptr(), ws.numel()) if ws is not None else (None, 0)
     if x2 is not None:
-        _lib.check(L.kyb_gemv_glu_t16(_fmt(fmt), t16.data_ptr(), n, k, x.data_ptr(), x2.data_ptr(), float(limit or 0.0), m, x.stride(0), float(gscale), y.data_ptr(), y.stride(0),
-                                      wp, wn, 1 if chained else 0, _stream()))
-        return y
-    _lib.check(L.kyb_gemv_t16(_fmt(fmt), t16.data_ptr(), n, k, x.data_ptr(), m, x.stride(0), float(gscale), y.data_ptr(), y.stride(0), wp, wn, 1 if chained else 0, _stream()))
+        rc = L.kyb_gemv_glu_t16(fid, t16.data_ptr(), n, k, x.data_ptr(), x2.data_ptr(), float(limit or 0.0), m, x.stride(0), float(gscale), y.data_ptr(), y.stride(0), wp, wn,
+                                1 if chained else 0, _stream())
+    else:
+        rc = L.kyb_gemv_t16(fid, t16.data_ptr(), n, k, x.data_ptr(), m, x.stride(0), float(gscale), y.data_ptr(), y.stride(0), wp, wn, 1 if chained else 0, _stream())
+    if rc:
+        _lib.check(rc)
     return y
 
 
@@ -360,7 +368,7 @@ def gemm_kq(fmt, t16: torch.Tensor, n: int, k: int, a: torch.Tensor, gscale: flo
     if a.stride(1) != 1:
         a = a.contiguous()
     m = a.shape[0]
-    d = out if out is not None else torch.empty((m, n), dtype=torch.float16, device=a.device)
+    d = out if out is not None else a.new_empty((m, n))
     L = _lib.lib()
     if split is None:
         split = L.kyb_gemm_kq_split(_fmt(fmt), n, k, m) if (msub == 0 and F.GEMM_SPLIT_K) else 1
