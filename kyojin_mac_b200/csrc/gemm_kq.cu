@@ -897,15 +897,16 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_kq_kernel(const __grid_con
         if (more) {
             // Software pipeline over the 64-input quarters: while the tensor-memory store of quarter P is on its way, the registers of quarter P + 1 are computed; the
             // wait for a free stage, the scale loads and the arithmetic overlap it.
+            // The refills are unconditional (behind the last tile they read it once more, and what is computed from it is not stored): fewer branches and copies.
             KqTile<FMT> tr;
             uint32_t r[16];
             kq_load<FMT>(wk.ptr, lane, tr);
             kq_prep_scales<FMT>(tr, scr, lane);
             __syncwarp();
             wk.advance(p, num_items, stride, rank, tord, kp, q, half);
-            if (wk.ok) kq_refill_scales<FMT>(wk.ptr, lane, tr);
+            kq_refill_scales<FMT>(wk.ptr, lane, tr);
             kq_compute_quarter<FMT, 0>(tr, scr, lane, r);
-            if (wk.ok) kq_refill<FMT, 0>(wk.ptr, lane, tr);
+            kq_refill<FMT, 0>(wk.ptr, lane, tr);
 #define KYB_KQ_WAIT(H)                                                               \
     {                                                                                \
         if (!mbar_wait_fast(empty + 8 * (H), parity)) failed = true;                 \
@@ -926,29 +927,23 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_kq_kernel(const __grid_con
                 KYB_KQ_WAIT(0)
                 tmem_st_16x256b_x4(tw, r);
                 kq_compute_quarter<FMT, 1>(tr, scr, lane, r);
-                if (more) kq_refill<FMT, 1>(wk.ptr, lane, tr);
+                kq_refill<FMT, 1>(wk.ptr, lane, tr);
                 tmem_st_16x256b_x4(tw + 32u, r);
                 KYB_KQ_PUBLISH(0)
                 kq_compute_quarter<FMT, 2>(tr, scr, lane, r);
-                if (more) kq_refill<FMT, 2>(wk.ptr, lane, tr);
+                kq_refill<FMT, 2>(wk.ptr, lane, tr);
                 KYB_KQ_WAIT(1)
                 tmem_st_16x256b_x4(tw + 64u, r);
                 kq_compute_quarter<FMT, 3>(tr, scr, lane, r);
-                if (more) kq_refill<FMT, 3>(wk.ptr, lane, tr);
+                kq_refill<FMT, 3>(wk.ptr, lane, tr);
                 tmem_st_16x256b_x4(tw + 96u, r);
                 KYB_KQ_PUBLISH(1)                                                       // its warp barrier also ends every lane's reads of this tile's scales
-                if (more) {
-                    kq_prep_scales<FMT>(tr, scr, lane);                                 // tr.sc holds the next tile's scale bytes
-                    __syncwarp();
-                    kq_compute_quarter<FMT, 0>(tr, scr, lane, r);                       // quarter 0 of the next tile
-                }
-                if (more) {
-                    wk.advance(p, num_items, stride, rank, tord, kp, q, half);
-                    if (wk.ok) {
-                        kq_refill_scales<FMT>(wk.ptr, lane, tr);
-                        kq_refill<FMT, 0>(wk.ptr, lane, tr);
-                    }
-                }
+                kq_prep_scales<FMT>(tr, scr, lane);                                     // tr.sc holds the next tile's scale bytes
+                __syncwarp();
+                kq_compute_quarter<FMT, 0>(tr, scr, lane, r);                           // quarter 0 of the next tile
+                if (more) wk.advance(p, num_items, stride, rank, tord, kp, q, half);
+                kq_refill_scales<FMT>(wk.ptr, lane, tr);
+                kq_refill<FMT, 0>(wk.ptr, lane, tr);
                 parity ^= 1u;
             }
 #undef KYB_KQ_WAIT
