@@ -13,6 +13,7 @@
 // result of an activation row does not depend on how many rows ride along.
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -1025,19 +1026,33 @@ int canonical_chunk(int ntiles, int nb) {
     return best;
 }
 
-// Warps per CTA, k-parts and the way work is dealt. k is split over CTAs only as far as the staged activations of a part must fit in shared memory next to the
-// warps' rings. For every warp count two ways are scored by how even the busiest warp's share is: whole row tiles per warp (nothing goes through the workspace)
-// or runs of chunks (chunk sums through the workspace and a finalize launch); more warps per SM are mildly preferred. Small matrices that would take the second
-// way are then moved to whole row tiles per CTA with the chunk sums in shared memory (one launch), see the end of the function.
+// Warps per CTA, k-parts and the way work is dealt: the launch that a small cost model (microseconds) finds cheapest.
+//   stream   the tiles at 5.6 TB/s or at the issue rate of a tile (about 115 / 220 / 400 clocks of an SM for one / two / four column tiles), divided by how even the
+//            shares of the warps are (whole row tiles: form (a), one k-part; runs of chunks: form (b); the square root, because the other warps of an SM run faster
+//            when one has finished) and of the CTAs (whole row tiles per CTA: form (c)), by the share of SMs in use and by an occupancy factor: 12 warps (three
+//            per scheduler) measured best for up to 16 rows, 14 and 16 lose 8-10 % again, 10 and fewer lose to latency
+//   staging  every CTA stages the activations of its k-part before its first tile: 0.022 us per 256 inputs and row measured, 0.085 us with the gated activation
+//            formed on the way (the plan does not know which, 0.027 is taken). So form (b) cuts k into as many parts as leave the SMs evenly used: Q6_K 5120 x 27648,
+//            eight rows, 3 parts of 36 blocks and 10 warps -> 18 parts of 6 blocks and 12 warps: 38.1 -> 30.3 us, gated 59.3 -> 33.0 us; one row 31.4 -> 27.3, gated
+//            38.9 -> 30.0 us
+//   finish   form (b): the chunk sums through the workspace (written and read at 4 TB/s) and about 3.5 us for the finalize launch inside a chain
 GemvPlan search_plan(int fmt, int64_t n, int64_t k, int64_t m) {
     const int sms = device_sms();
     const int nb = (int)(k / 256), ntiles = (int)((n + 15) / 16);
     const size_t smem_cap = 226 * 1024;
     const int kc = canonical_chunk(ntiles, nb), nchunks = (nb + kc - 1) / kc;
     const int v = variant_of(m), nt = VAR_NT[v], mst = VAR_MST[v];
-    const int max_warps = nt <= 2 ? 12 : 8;                            // measured: 13 to 16 warps per SM are slower than 10 to 12 on every shape
+    const int max_warps = nt <= 2 ? 12 : 8;
+    const double tiles = (double)ntiles * nb, tile_clk = nt == 1 ? 115.0 : nt == 2 ? 220.0 : 400.0;
+    const double stream_us = std::max(tiles * (double)kyb_tile_bytes(fmt) / 5.6e6, tiles * tile_clk / sms / 1900.0);
+    static const double OCC[13] = {0.0, 0.3, 0.4, 0.5, 0.60, 0.62, 0.68, 0.74, 0.82, 0.84, 0.90, 0.93, 1.0};
+    auto occupancy = [&](int warps) { return nt <= 2 ? OCC[warps] : std::min(1.0, 0.52 + 0.06 * warps); };
+    auto staging_us = [&](int blocks) { return 0.027 * blocks * (double)m; };
+    // a warp works through its tiles one after the other: about 0.42 us per tile even when the SM is nearly empty (more with more column tiles)
+    auto serial_us = [&](double rounds, int tiles_each) { return rounds * tiles_each * (nt == 1 ? 0.42 : nt == 2 ? 0.55 : 0.9); };
+    const double finish_us = 3.5 + (double)nchunks * (double)m * (double)n * 8.0 / 4.0e6;
     GemvPlan best{};
-    double best_score = -1.0;
+    double best_us = 0.0;
     for (int ksplit = 1; ksplit <= std::min(nchunks, sms); ++ksplit) {
         const int cpp = (nchunks + ksplit - 1) / ksplit;
         if ((nchunks + cpp - 1) / cpp != ksplit) continue;               // one representative per distinct split
@@ -1047,36 +1062,34 @@ GemvPlan search_plan(int fmt, int64_t n, int64_t k, int64_t m) {
             if (smem > smem_cap) continue;
             const double wp = (double)(grid / ksplit) * warps;                                  // warps of a part
             const double parts = (double)nchunks / ((double)ksplit * cpp);                      // the last part may be shorter
-            // measured on every shape of the benchmark: 10 to 12 warps per SM are within 2 % of each other when their busiest warps carry the same load,
-            // fewer than 9 or more than 12 are slower; fewer are taken only when shared memory leaves no choice (many activation rows)
-            const int pref = nt <= 2 ? 10 : 6;
-            const double occupancy = warps >= pref ? 1.0 : 0.45 + 0.05 * warps;
-            const double common = parts * ((double)grid / sms) * occupancy * (1.0 - 0.02 * (ksplit - 1));
+            const double common = parts * ((double)grid / sms) * occupancy(warps);
             for (int aligned = 0; aligned < 2; ++aligned) {
                 const double upw = aligned ? ntiles / wp : (double)ntiles * cpp / wp;           // row tiles or units per warp
-                const double balance = upw / std::ceil(upw);
-                const double shared = aligned && ksplit == 1 ? 1.0 : 0.9;                       // cost of the workspace round trip and the finalize launch
-                const double score = balance * common * shared;
-                if (score > best_score) best_score = score, best = GemvPlan{nt, mst, warps, kyb::GEMV_DSTAGES, kbp, ksplit, grid, smem, kc, nchunks, cpp, aligned, 0};
+                const double balance = std::sqrt(upw / std::ceil(upw));
+                const double us = std::max(stream_us / (balance * common), serial_us(std::ceil(upw), aligned ? kbp : kc)) + staging_us(kbp) + (aligned && ksplit == 1 ? 0.0 : finish_us);
+                if (best.warps == 0 || us < best_us) best_us = us, best = GemvPlan{nt, mst, warps, kyb::GEMV_DSTAGES, kbp, ksplit, grid, smem, kc, nchunks, cpp, aligned, 0};
             }
         }
-        if (best_score > 0) break;                                        // the smallest split that fits
     }
-    // Form (c) instead of form (b) where the second launch costs more than the uneven shares of whole row tiles per CTA: G = min(SMs, row tiles) CTAs own
-    // floor / ceil (row tiles / G) row tiles each, so the product runs as long as its busiest CTA; against that stand about 2.5 us for the finalize launch of form (b)
-    // (measured inside chained launches: 4096 x 4096 7.4 -> 5.2 us, 10240 x 5120 10.2 -> 9.1 us, 5120 x 8192 9.3 -> 8.7 us at one row; more with 8 rows).
-    // The whole of k is staged in every CTA, so up to 8 activation rows and only while that fits shared memory; at least 64 CTAs must get work.
-    if (best.warps > 0 && !(best.aligned && best.ksplit == 1) && ntiles >= 64 && m <= 8) {
+    // Form (c): CTA c owns whole row tiles (the product runs as long as the CTA with the most), the whole of k is staged in every CTA, so up to 8 activation rows and
+    // only while that fits shared memory; at least 64 CTAs must get work. It needs no second launch: taken instead of form (b) while the uneven shares of the CTAs
+    // cost less than 2.5 us (4096 x 4096, one row 7.4 -> 5.2 us, with the warp count that deals the chunks evenly 4.3 us; 10240 x 5120 10.2 -> 9.6; 5120 x 8192
+    // 9.3 -> 9.1), and instead of form (a) where the model says so.
+    if (best.warps > 0 && ntiles >= 64 && m <= 8) {
         const int grid = std::min(sms, ntiles), rpc = (ntiles + grid - 1) / grid;
-        const double t_us = (double)ntiles * nb * (double)kyb_tile_bytes(fmt) / 5.0e6;          // the product at 5 TB/s
-        const double penalty_us = t_us * ((double)rpc * grid / ntiles - 1.0);
         const size_t cpart = (size_t)rpc * nchunks * (size_t)m * 16 * sizeof(float);
-        if (penalty_us < 2.5) {
-            for (int warps = max_warps; warps >= 8; --warps) {
-                const size_t smem = plan_smem(fmt, nt, mst, nb, warps, kyb::GEMV_DSTAGES) + cpart;
-                if (smem <= smem_cap) return GemvPlan{nt, mst, warps, kyb::GEMV_DSTAGES, nb, 1, grid, smem, kc, nchunks, nchunks, 0, 1};
-            }
+        const double even = (double)ntiles / ((double)rpc * grid), t_us = tiles * (double)kyb_tile_bytes(fmt) / 5.0e6;
+        const bool few = !(best.aligned && best.ksplit == 1) && t_us * (1.0 / even - 1.0) < 2.5;
+        GemvPlan c{};
+        double c_us = 0.0;
+        for (int warps = max_warps; warps >= 8; --warps) {
+            const size_t smem = plan_smem(fmt, nt, mst, nb, warps, kyb::GEMV_DSTAGES) + cpart;
+            if (smem > smem_cap) continue;
+            const double upw = (double)rpc * nchunks / warps, balance = even * std::sqrt(upw / std::ceil(upw));
+            const double us = std::max(stream_us / (balance * ((double)grid / sms) * occupancy(warps)), serial_us(std::ceil(upw), kc)) + staging_us(nb);
+            if (c.warps == 0 || us < c_us) c_us = us, c = GemvPlan{nt, mst, warps, kyb::GEMV_DSTAGES, nb, 1, grid, smem, kc, nchunks, nchunks, 0, 1};
         }
+        if (c.warps > 0 && (few || c_us < best_us)) return c;
     }
     return best;
 }

@@ -1,0 +1,43 @@
+"""The launch planner of the decode product: every plan of the accepted range is one the kernel can run (no GPU needed), and products over shapes whose plans differ most
+give the same bits as the exposed chunk sums, row for row whatever the number of rows (GPU)."""
+import random
+
+import pytest
+import torch
+
+from kyojin_mac_b200 import ops, synth
+from kyojin_mac_b200.layout import FMT_ID
+
+KC_MAX, SMEM_MAX, SMS = 8, 226 * 1024, 148
+
+
+@pytest.mark.parametrize("fmt", sorted(FMT_ID))
+def test_plans_are_runnable(fmt):
+    rng = random.Random(FMT_ID[fmt])
+    for _ in range(300):
+        n, nb, m = int(2 ** rng.uniform(0, 17)), int(2 ** rng.uniform(0, 9)), rng.randint(1, 32)
+        p = ops.gemv_plan(fmt, n, nb * 256, m)
+        where = (fmt, n, nb * 256, m, p)
+        assert 4 <= p["warps"] <= 12 and p["warps"] * 32 <= (512 if p["nt"] <= 2 else 256) and p["smem"] <= SMEM_MAX, where
+        assert 8 * p["nt"] >= m and 1 <= p["kc"] <= KC_MAX and p["grid"] <= SMS, where
+        assert p["kbp"] * p["ksplit"] >= nb and p["kbp"] * (p["ksplit"] - 1) < nb and p["grid"] % p["ksplit"] == 0, where   # the parts cover k and none is empty
+        assert p["kbp"] == nb or p["kbp"] % p["kc"] == 0, where                              # a part is whole chunks
+        assert (ops.gemv_workspace_bytes(fmt, n, nb * 256, m) > 0) == (p["aligned"] == 0 or (p["aligned"] == 1 and p["ksplit"] > 1)), where
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt,n,k", [("q6_k", 1577, 6912), ("q4_k", 609, 5120), ("q5_k", 4100, 8192), ("q3_k", 865, 5888), ("nvfp4", 2400, 1280), ("q8_0", 33, 13568)])
+def test_rows_do_not_depend_on_the_plan(fmt, n, k):
+    from kyojin_mac_b200 import mma_gemv
+    from kyojin_mac_b200.foreign_linear import DevPack
+    dev = DevPack.from_t16(fmt, synth.t16_random_device(fmt, n, k, seed=5), n, k)
+    g = torch.Generator(device="cuda").manual_seed(6)
+    x, x2 = ((torch.randn((32, k), device="cuda", generator=g) * 0.5).to(torch.float16) for _ in range(2))
+    want = mma_gemv.finalize_rows(dev, mma_gemv.partial_mma(dev, x, 32), 32)
+    gated = ops.gemv(fmt, dev.t16, n, k, ops.silu_mul(x, x2))
+    ref = x.double() @ dev.dequant(torch.float32).double().T
+    assert ((want.double() - ref).norm() / ref.norm()).item() <= 1e-3
+    for m in (1, 2, 4, 7, 8, 9, 16, 17, 32):
+        assert torch.equal(ops.gemv(fmt, dev.t16, n, k, x[:m]), want[:m]), (m, ops.gemv_plan(fmt, n, k, m))
+        assert torch.equal(ops.gemv(fmt, dev.t16, n, k, x[:m], x2=x2[:m]), gated[:m]), (m, ops.gemv_plan(fmt, n, k, m))
+    ops.check_device_status()
