@@ -576,10 +576,18 @@ __global__ void moe_groups_kernel(const uint32_t* __restrict__ eids, int S, int 
 // k order; (c) small matrices, where a second launch would cost as much as the product: CTA c owns the row tiles [ntiles c / G, ntiles (c + 1) / G), its warps
 // share the chunks of those row tiles as in (b), the chunk sums go to shared memory and after a CTA barrier the threads add them in k order and store y.
 // Either way an output is the left-to-right sum of the same chunk sums, so results do not depend on the batch size, the grid or the split.
+// Threads a CTA may have, which is what its registers are divided by: 128 registers up to two column tiles (see below); 168 for three and four, except for the formats
+// whose tile takes 20 to 32 registers, which spill or lose 5-10 % with four column tiles in 168 registers and run 8 warps of 255 instead. Three column tiles for 17 to
+// 24 rows, against four: Q4_K 27648 x 5120, 20 rows 51.5 -> 40.0 us, Q6_K 32001 x 4096 54.5 -> 49.4, Q3_K 5075 x 11008 30.5 -> 24.1; four column tiles with 12 warps
+// instead of 8: Q4_K 27648 x 5120, 32 rows 54.7 -> 49.6 us.
+__host__ __device__ constexpr int gemv_threads(int fmt, int nt) {
+    return nt <= 2 ? 512 : nt == 4 && (fmt == KYB_FMT_Q5_K || fmt == KYB_FMT_Q6_K || fmt == KYB_FMT_Q8_0) ? 256 : 384;
+}
+
 template <int FMT, int NT, int MST>
 // At most 16 warps per CTA: 128 registers per thread let the compiler keep the unpacked operands of several MMAs in flight (with 24 warps and 80 registers the
 // kernel spilled and its steady rate was 15 % lower).
-__global__ void __launch_bounds__(NT <= 2 ? 512 : 256, 1) gemv_t16_kernel(const GemvParams p) {
+__global__ void __launch_bounds__(gemv_threads(FMT, NT), 1) gemv_t16_kernel(const GemvParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int TB = kyb_tile_bytes(FMT);
     constexpr int CS = NT * MST * 32;
@@ -969,10 +977,10 @@ size_t plan_smem(int fmt, int nt, int mst, int kbp, int warps, int stages) {
 }
 
 // kernel variants: (column tiles, staged activation rows per tile)
-constexpr int NVAR = 6;
-constexpr int VAR_NT[NVAR] = {1, 1, 1, 1, 2, 4}, VAR_MST[NVAR] = {1, 2, 4, 8, 8, 8};
+constexpr int NVAR = 7;
+constexpr int VAR_NT[NVAR] = {1, 1, 1, 1, 2, 3, 4}, VAR_MST[NVAR] = {1, 2, 4, 8, 8, 8, 8};
 
-int variant_of(int64_t m) { return m <= 1 ? 0 : m <= 2 ? 1 : m <= 4 ? 2 : m <= 8 ? 3 : m <= 16 ? 4 : 5; }
+int variant_of(int64_t m) { return m <= 1 ? 0 : m <= 2 ? 1 : m <= 4 ? 2 : m <= 8 ? 3 : m <= 16 ? 4 : m <= 24 ? 5 : 6; }
 
 template <int FMT>
 const void* kernel_of_fmt(int v) {
@@ -982,6 +990,7 @@ const void* kernel_of_fmt(int v) {
         case 2: return (const void*)kyb::gemv_t16_kernel<FMT, 1, 4>;
         case 3: return (const void*)kyb::gemv_t16_kernel<FMT, 1, 8>;
         case 4: return (const void*)kyb::gemv_t16_kernel<FMT, 2, 8>;
+        case 5: return (const void*)kyb::gemv_t16_kernel<FMT, 3, 8>;
         default: return (const void*)kyb::gemv_t16_kernel<FMT, 4, 8>;
     }
 }
@@ -1027,7 +1036,7 @@ int canonical_chunk(int ntiles, int nb) {
 }
 
 // Warps per CTA, k-parts and the way work is dealt: the launch that a small cost model (microseconds) finds cheapest.
-//   stream   the tiles at 5.6 TB/s or at the issue rate of a tile (about 115 / 220 / 400 clocks of an SM for one / two / four column tiles), divided by how even the
+//   stream   the tiles at 5.6 TB/s or at the issue rate of a tile (about 115 / 220 / 310 / 400 clocks of an SM for one to four column tiles), divided by how even the
 //            shares of the warps are (whole row tiles: form (a), one k-part; runs of chunks: form (b); the square root, because the other warps of an SM run faster
 //            when one has finished) and of the CTAs (whole row tiles per CTA: form (c)), by the share of SMs in use and by an occupancy factor: 12 warps (three
 //            per scheduler) measured best for up to 16 rows, 14 and 16 lose 8-10 % again, 10 and fewer lose to latency
@@ -1042,14 +1051,14 @@ GemvPlan search_plan(int fmt, int64_t n, int64_t k, int64_t m) {
     const size_t smem_cap = 226 * 1024;
     const int kc = canonical_chunk(ntiles, nb), nchunks = (nb + kc - 1) / kc;
     const int v = variant_of(m), nt = VAR_NT[v], mst = VAR_MST[v];
-    const int max_warps = nt <= 2 ? 12 : 8;
-    const double tiles = (double)ntiles * nb, tile_clk = nt == 1 ? 115.0 : nt == 2 ? 220.0 : 400.0;
+    const int max_warps = std::min(12, kyb::gemv_threads(fmt, nt) / 32);
+    const double tiles = (double)ntiles * nb, tile_clk = nt == 1 ? 115.0 : nt == 2 ? 220.0 : nt == 3 ? 310.0 : 400.0;
     const double stream_us = std::max(tiles * (double)kyb_tile_bytes(fmt) / 5.6e6, tiles * tile_clk / sms / 1900.0);
     static const double OCC[13] = {0.0, 0.3, 0.4, 0.5, 0.60, 0.62, 0.68, 0.74, 0.82, 0.84, 0.90, 0.93, 1.0};
-    auto occupancy = [&](int warps) { return nt <= 2 ? OCC[warps] : std::min(1.0, 0.52 + 0.06 * warps); };
+    auto occupancy = [&](int warps) { return max_warps == 8 ? std::min(1.0, 0.52 + 0.06 * warps) : OCC[warps]; };
     auto staging_us = [&](int blocks) { return 0.027 * blocks * (double)m; };
     // a warp works through its tiles one after the other: about 0.42 us per tile even when the SM is nearly empty (more with more column tiles)
-    auto serial_us = [&](double rounds, int tiles_each) { return rounds * tiles_each * (nt == 1 ? 0.42 : nt == 2 ? 0.55 : 0.9); };
+    auto serial_us = [&](double rounds, int tiles_each) { return rounds * tiles_each * (nt == 1 ? 0.42 : nt == 2 ? 0.55 : nt == 3 ? 0.72 : 0.9); };
     const double finish_us = 3.5 + (double)nchunks * (double)m * (double)n * 8.0 / 4.0e6;
     GemvPlan best{};
     double best_us = 0.0;

@@ -18,7 +18,7 @@ def test_plans_are_runnable(fmt):
         n, nb, m = int(2 ** rng.uniform(0, 17)), int(2 ** rng.uniform(0, 9)), rng.randint(1, 32)
         p = ops.gemv_plan(fmt, n, nb * 256, m)
         where = (fmt, n, nb * 256, m, p)
-        assert 4 <= p["warps"] <= 12 and p["warps"] * 32 <= (512 if p["nt"] <= 2 else 256) and p["smem"] <= SMEM_MAX, where
+        assert 4 <= p["warps"] <= 12 and p["warps"] * 32 <= (512 if p["nt"] <= 2 else 384 if p["nt"] == 3 or fmt not in ("q5_k", "q6_k", "q8_0") else 256) and p["smem"] <= SMEM_MAX, where
         assert 8 * p["nt"] >= m and 1 <= p["kc"] <= KC_MAX and p["grid"] <= SMS, where
         assert p["kbp"] * p["ksplit"] >= nb and p["kbp"] * (p["ksplit"] - 1) < nb and p["grid"] % p["ksplit"] == 0, where   # the parts cover k and none is empty
         assert p["kbp"] == nb or p["kbp"] % p["kc"] == 0, where                              # a part is whole chunks
@@ -37,7 +37,7 @@ def test_rows_do_not_depend_on_the_plan(fmt, n, k):
     gated = ops.gemv(fmt, dev.t16, n, k, ops.silu_mul(x, x2))
     ref = x.double() @ dev.dequant(torch.float32).double().T
     assert ((want.double() - ref).norm() / ref.norm()).item() <= 1e-3
-    for m in (1, 2, 4, 7, 8, 9, 16, 17, 32):
+    for m in (1, 2, 4, 7, 8, 9, 16, 17, 24, 25, 32):
         assert torch.equal(ops.gemv(fmt, dev.t16, n, k, x[:m]), want[:m]), (m, ops.gemv_plan(fmt, n, k, m))
         assert torch.equal(ops.gemv(fmt, dev.t16, n, k, x[:m], x2=x2[:m]), gated[:m]), (m, ops.gemv_plan(fmt, n, k, m))
     ops.check_device_status()
