@@ -410,6 +410,83 @@ __global__ void __launch_bounds__(512) router_logits_kernel(const XT* __restrict
     }
 }
 
+// The same for few tokens (decode), where the walk along a weight row is one load latency after the other: two rows per warp instead of four spread the rows over
+// twice the warps, and the weights of the next D steps are in flight while D steps are summed (one step at a time: 55 us for 64 tokens, 257 x 7168; now 13 us).
+// The sums are formed in the same order.
+template <typename XT, int TT>
+__global__ void __launch_bounds__(256) router_logits_few_kernel(const XT* __restrict__ x, int64_t ldx, const float* __restrict__ gw, const float* __restrict__ sgw, int T, int E, int H,
+                                                                float* __restrict__ lg, int64_t ldl) {
+    extern __shared__ __align__(16) unsigned char router_smem[];
+    XT* xs = reinterpret_cast<XT*>(router_smem);
+    constexpr int PER = 16 / (int)sizeof(XT), RE = 2, D = 8;
+    const int t0 = blockIdx.x * TT, H4 = H / 4;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, R = E + (sgw ? 1 : 0), nw = blockDim.x >> 5;
+    int r0 = (blockIdx.y * nw + warp) * RE;
+    const float4* wp[RE];
+    float4 nxt[D][RE];
+    auto rows = [&]() {
+#pragma unroll
+        for (int e = 0; e < RE; ++e) {
+            const int r = min(r0 + e, R - 1);                               // a short last group repeats its last row; the repeats are not stored
+            wp[e] = reinterpret_cast<const float4*>(r < E ? gw + (size_t)r * H : sgw);
+        }
+    };
+    auto fetch = [&](int i0) {
+#pragma unroll
+        for (int d = 0; d < D; ++d)
+#pragma unroll
+            for (int e = 0; e < RE; ++e) nxt[d][e] = __ldg(wp[e] + min(i0 + 32 * d, H4 - 1));   // past the end: a repeated load whose value is not used
+    };
+    if (r0 < R) rows(), fetch(lane);                                        // the first weights travel while the tokens are staged
+    for (int j = 0; j < TT; ++j) {                                          // asynchronous copies: all of them are in flight at once
+        const XT* src = x + (size_t)min(t0 + j, T - 1) * ldx;               // rows past T repeat the last token; their results are not stored
+        for (int c = threadIdx.x; c < H / PER; c += blockDim.x)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(xs + (size_t)j * H + (size_t)c * PER)), "l"(src + (size_t)c * PER) : "memory");
+    }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    while (r0 < R) {
+        unsigned long long acc[RE][TT];
+#pragma unroll
+        for (int e = 0; e < RE; ++e)
+#pragma unroll
+            for (int j = 0; j < TT; ++j) acc[e][j] = 0ull;
+        for (int i0 = lane; i0 < H4; i0 += 32 * D) {
+            float4 w[D][RE];
+#pragma unroll
+            for (int d = 0; d < D; ++d)
+#pragma unroll
+                for (int e = 0; e < RE; ++e) w[d][e] = nxt[d][e];
+            fetch(i0 + 32 * D);
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+                const int i = i0 + 32 * d;
+                if (i < H4) {
+#pragma unroll
+                    for (int j = 0; j < TT; ++j) {
+                        const float4 v = XVec4<XT>::ld(xs + (size_t)j * H + 4 * i);
+                        const unsigned long long vlo = pack2(v.x, v.y), vhi = pack2(v.z, v.w);
+#pragma unroll
+                        for (int e = 0; e < RE; ++e) acc[e][j] = ffma2(pack2(w[d][e].z, w[d][e].w), vhi, ffma2(pack2(w[d][e].x, w[d][e].y), vlo, acc[e][j]));
+                    }
+                }
+            }
+        }
+        const int r1 = r0;
+        r0 += gridDim.y * nw * RE;
+        if (r0 < R) rows(), fetch(lane);
+#pragma unroll
+        for (int e = 0; e < RE; ++e)
+#pragma unroll
+            for (int j = 0; j < TT; ++j) {
+                float v = sum2(acc[e][j]);
+#pragma unroll
+                for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == 0 && t0 + j < T && r1 + e < R) lg[(size_t)(t0 + j) * ldl + r1 + e] = v;
+            }
+    }
+}
+
 // The same product with the roles exchanged, for many tokens: a CTA keeps WR weight rows (fp32) in shared memory and its warps stream token rows, RE per pass,
 // so a token row read from L2 serves WR weight rows and the L2 reads fall from (T / 8) x |weights| to (R / WR) x |tokens|. Every logit is summed in the same
 // order as in router_logits_kernel (pairs over even and odd inputs per lane, lanes combined by the same shuffles), so the two kernels agree bit for bit.
@@ -588,8 +665,21 @@ static int launch_router(const void* x, int64_t ldx, const float* gw, const floa
         configured = true;
     }
     const int64_t gx = (T + TT - 1) / TT;
+    const int R = E + (sgw ? 1 : 0);
+    if (T <= 128) {
+        // few tokens (at 300 the other kernel, which reads a weight row for four rows' worth of staged tokens, is faster: 62 us against 104): the weight rows are dealt two by two to the warps of as many CTAs as there are SMs (4 warps per CTA while that still leaves SMs without one)
+        static bool few_configured = false;
+        if (!few_configured) {
+            KYB_CUDA(cudaFuncSetAttribute(kyb::router_logits_few_kernel<XT, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+            few_configured = true;
+        }
+        const int warps = gx * ((R + 15) / 16) <= 74 ? 4 : 8;
+        const int64_t gy = std::min<int64_t>((R + 2 * warps - 1) / (2 * warps), std::max<int64_t>(1, (148 + gx / 2) / gx));
+        kyb::router_logits_few_kernel<XT, TT><<<dim3((unsigned)gx, (unsigned)gy), warps * 32, smem, st>>>((const XT*)x, ldx, gw, sgw, (int)T, E, (int)H, lg, ldl);
+        return kyb_launch_check("router_logits_few");
+    }
     const int threads = T >= 1024 ? 512 : 256;                               // many tokens: 16 warps per CTA hide the L2 latency of the weight rows
-    const int R = E + (sgw ? 1 : 0), ymax = (R + threads / 8 - 1) / (threads / 8);   // warps x 4 rows per pass
+    const int ymax = (R + threads / 8 - 1) / (threads / 8);   // warps x 4 rows per pass
     const int gy = (int)std::min<int64_t>(ymax, std::max<int64_t>(1, (2 * 148 + gx - 1) / gx));   // few tokens: spread the weight rows over more CTAs
     kyb::router_logits_kernel<XT, TT><<<dim3((unsigned)gx, (unsigned)gy), threads, smem, st>>>((const XT*)x, ldx, gw, sgw, (int)T, E, (int)H, lg, ldl);
     return kyb_launch_check("router_logits");
