@@ -1045,7 +1045,8 @@ int canonical_chunk(int ntiles, int nb) {
 //            eight rows, 3 parts of 36 blocks and 10 warps -> 18 parts of 6 blocks and 12 warps: 38.1 -> 30.3 us, gated 59.3 -> 33.0 us; one row 31.4 -> 27.3, gated
 //            38.9 -> 30.0 us
 //   finish   form (b): the chunk sums through the workspace (written and read at 4 TB/s) and about 3.5 us for the finalize launch inside a chain
-GemvPlan search_plan(int fmt, int64_t n, int64_t k, int64_t m) {
+// sums: chunk sums may go through a workspace; without, only form (a) over one k-part and form (c) are left (no warps in the plan: neither fits).
+GemvPlan search_plan(int fmt, int64_t n, int64_t k, int64_t m, bool sums) {
     const int sms = device_sms();
     const int nb = (int)(k / 256), ntiles = (int)((n + 15) / 16);
     const size_t smem_cap = 226 * 1024;
@@ -1073,6 +1074,7 @@ GemvPlan search_plan(int fmt, int64_t n, int64_t k, int64_t m) {
             const double parts = (double)nchunks / ((double)ksplit * cpp);                      // the last part may be shorter
             const double common = parts * ((double)grid / sms) * occupancy(warps);
             for (int aligned = 0; aligned < 2; ++aligned) {
+                if (!(aligned && ksplit == 1) && !sums) continue;
                 const double upw = aligned ? ntiles / wp : (double)ntiles * cpp / wp;           // row tiles or units per warp
                 const double balance = std::sqrt(upw / std::ceil(upw));
                 const double us = std::max(stream_us / (balance * common), serial_us(std::ceil(upw), aligned ? kbp : kc)) + staging_us(kbp) + (aligned && ksplit == 1 ? 0.0 : finish_us);
@@ -1084,7 +1086,7 @@ GemvPlan search_plan(int fmt, int64_t n, int64_t k, int64_t m) {
     // only while that fits shared memory; at least 64 CTAs must get work. It needs no second launch: taken instead of form (b) while the uneven shares of the CTAs
     // cost less than 2.5 us (4096 x 4096, one row 7.4 -> 5.2 us, with the warp count that deals the chunks evenly 4.3 us; 10240 x 5120 10.2 -> 9.6; 5120 x 8192
     // 9.3 -> 9.1), and instead of form (a) where the model says so.
-    if (best.warps > 0 && ntiles >= 64 && m <= 8) {
+    if ((best.warps > 0 || !sums) && ntiles >= 64 && m <= 8) {
         const int grid = std::min(sms, ntiles), rpc = (ntiles + grid - 1) / grid;
         const size_t cpart = (size_t)rpc * nchunks * (size_t)m * 16 * sizeof(float);
         const double even = (double)ntiles / ((double)rpc * grid), t_us = tiles * (double)kyb_tile_bytes(fmt) / 5.0e6;
@@ -1103,15 +1105,15 @@ GemvPlan search_plan(int fmt, int64_t n, int64_t k, int64_t m) {
     return best;
 }
 
-// plans are cached per (format, n, k, m): a decode step calls this per linear
-GemvPlan make_plan(int fmt, int64_t n, int64_t k, int64_t m) {
+// plans are cached per (format, n, k, m, chunk sums allowed): a decode step calls this per linear
+GemvPlan make_plan(int fmt, int64_t n, int64_t k, int64_t m, bool sums = true) {
     static std::mutex mu;
-    static std::map<std::tuple<int, int64_t, int64_t, int64_t>, GemvPlan> cache;
-    const auto key = std::make_tuple(fmt, n, k, m);
+    static std::map<std::tuple<int, int64_t, int64_t, int64_t, bool>, GemvPlan> cache;
+    const auto key = std::make_tuple(fmt, n, k, m, sums);
     std::lock_guard<std::mutex> lk(mu);
     auto it = cache.find(key);
     if (it != cache.end()) return it->second;
-    const GemvPlan pl = search_plan(fmt, n, k, m);
+    const GemvPlan pl = search_plan(fmt, n, k, m, sums);
     cache.emplace(key, pl);
     return pl;
 }
@@ -1145,6 +1147,14 @@ int launch_maybe_chained(const void* kern, dim3 grid, dim3 block, size_t smem, c
 
 bool two_step(const GemvPlan& pl) { return !pl.local && !(pl.aligned && pl.ksplit == 1); }     // form (b): chunk sums through the workspace, then the finalize kernel
 size_t partial_bytes(const GemvPlan& pl, int64_t n, int64_t m) { return (size_t)pl.nchunks * (size_t)m * (size_t)((n + 15) / 16 * 16) * sizeof(float); }
+
+// the plan for a caller that brings `bytes` of scratch: where the best one needs more, a form without chunk sums in memory if there is one (the same bits)
+GemvPlan plan_within(int fmt, int64_t n, int64_t k, int64_t m, size_t bytes) {
+    const GemvPlan pl = make_plan(fmt, n, k, m);
+    if (pl.warps == 0 || !two_step(pl) || partial_bytes(pl, n, m) <= bytes) return pl;
+    const GemvPlan without = make_plan(fmt, n, k, m, false);
+    return without.warps > 0 ? without : pl;
+}
 
 int check_gemv_args(int fmt, const void* t16, int64_t n, int64_t k, const void* x, int64_t m, int64_t ldx) {
     KYB_REQUIRE(fmt >= 0 && fmt < KYB_FMT_COUNT, "unknown weight format %d", fmt);
@@ -1202,7 +1212,7 @@ extern "C" int kyb_gemv_t16(int fmt, const void* t16, int64_t n, int64_t k, cons
     if (int rc = check_gemv_args(fmt, t16, n, k, x, m, ldx)) return rc;
     KYB_REQUIRE(y && ldy >= n, "y is null or ldy=%lld < n", (long long)ldy);
     KYB_REQUIRE((flags & ~KYB_GEMV_CHAINED) == 0, "unknown flags 0x%x", flags);
-    const GemvPlan pl = make_plan(fmt, n, k, m);
+    const GemvPlan pl = plan_within(fmt, n, k, m, workspace && ((uintptr_t)workspace & 15) == 0 ? workspace_bytes : 0);
     KYB_REQUIRE(pl.warps > 0, "no launch configuration fits shared memory for k=%lld m=%lld", (long long)k, (long long)m);
     const size_t need = two_step(pl) ? partial_bytes(pl, n, m) : 0;
     if (need && (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 15))) {
@@ -1222,7 +1232,7 @@ extern "C" int kyb_gemv_glu_t16(int fmt, const void* t16, int64_t n, int64_t k, 
     KYB_REQUIRE(b && ((uintptr_t)b & 15) == 0, "b is null or not 16-byte aligned");
     KYB_REQUIRE(y && ldy >= n, "y is null or ldy=%lld < n", (long long)ldy);
     KYB_REQUIRE((flags & ~KYB_GEMV_CHAINED) == 0, "unknown flags 0x%x", flags);
-    const GemvPlan pl = make_plan(fmt, n, k, m);
+    const GemvPlan pl = plan_within(fmt, n, k, m, workspace && ((uintptr_t)workspace & 15) == 0 ? workspace_bytes : 0);
     KYB_REQUIRE(pl.warps > 0, "no launch configuration fits shared memory for k=%lld m=%lld", (long long)k, (long long)m);
     const size_t need = two_step(pl) ? partial_bytes(pl, n, m) : 0;
     if (need && (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 15))) {
@@ -1293,7 +1303,7 @@ extern "C" int kyb_gemv_t16_static(int fmt, const void* t16, int64_t n, int64_t 
                                    int check, void* stream) {
     if (int rc = check_gemv_args(fmt, t16, n, k, x, m, ldx)) return rc;
     KYB_REQUIRE(y && ldy >= n, "y is null or ldy=%lld < n", (long long)ldy);
-    const GemvPlan pl = make_plan(fmt, n, k, m);
+    const GemvPlan pl = plan_within(fmt, n, k, m, KYB_GEMV_STATIC_SCRATCH_BYTES);
     KYB_REQUIRE(pl.warps > 0, "no launch configuration fits shared memory for k=%lld m=%lld", (long long)k, (long long)m);
     const size_t need = two_step(pl) ? partial_bytes(pl, n, m) : 0;
     if (need > KYB_GEMV_STATIC_SCRATCH_BYTES) {

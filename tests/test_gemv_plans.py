@@ -41,3 +41,19 @@ def test_rows_do_not_depend_on_the_plan(fmt, n, k):
         assert torch.equal(ops.gemv(fmt, dev.t16, n, k, x[:m]), want[:m]), (m, ops.gemv_plan(fmt, n, k, m))
         assert torch.equal(ops.gemv(fmt, dev.t16, n, k, x[:m], x2=x2[:m]), gated[:m]), (m, ops.gemv_plan(fmt, n, k, m))
     ops.check_device_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt,n,k,m", [("q4_k", 9216, 2560, 12), ("q4_k", 9216, 2560, 24)])
+def test_products_without_a_workspace(fmt, n, k, m):
+    """A shape whose best plan uses a workspace although another form serves it: a caller without one gets that form, the same bits."""
+    from kyojin_mac_b200 import _lib
+    if ops.gemv_workspace_bytes(fmt, n, k, m) == 0:
+        pytest.skip("the best plan needs no workspace here")
+    t16 = synth.t16_random_device(fmt, n, k, seed=7)
+    x = torch.randn((m, k), device="cuda").to(torch.float16)
+    y = torch.empty((m, n), dtype=torch.float16, device="cuda")
+    L = _lib.lib()
+    rc = L.kyb_gemv_t16(ops._fmt(fmt), t16.data_ptr(), n, k, x.data_ptr(), m, x.stride(0), 1.0, y.data_ptr(), y.stride(0), None, 0, 0, ops._stream())
+    assert rc == 0, L.kyb_last_error()
+    assert torch.equal(y, ops.gemv(fmt, t16, n, k, x))
