@@ -1072,20 +1072,34 @@ int kq_launch(int fmt, const CUtensorMap& ta, const KybOutMaps& outs, kyb::KqPar
 
 // Activation rows per item (a multiple of 32, at most 256) for `tiles_n` column tiles on `units` CTAs or pairs: the whole rounds of equal items that cost least. A
 // stage of an item costs its MMAs (2 clocks per row) but never less than the decode of its weights (`dec` clocks), an item about 12 stages' worth of start and end.
+// The candidates are the item sizes, not the numbers of items, so any m has the same few of them and the widest one always counts.
 int kq_rows_per_item(int64_t m, int64_t tiles_n, int units, double stages, double dec, double* cost_out) {
     int best = 0;
     double best_cost = 0.0;
-    for (int tm = (int)((m + 255) / 256), last = 0; tm <= (int)((m + 31) / 32) && tm <= 4096; ++tm) {
-        const int mt = (int)((m + (int64_t)tm * 32 - 1) / ((int64_t)tm * 32)) * 32;
-        if (mt == last) continue;
-        last = mt;
+    for (int mt = 256; mt >= 32; mt -= 32) {
+        const int64_t tm = (m + mt - 1) / mt;
+        if ((m + tm * 32 - 1) / (tm * 32) * 32 != mt) continue;                        // as many items of fewer rows cover m: that size is the candidate
         if (mt < 96 && best) break;                                                    // narrower items are bound by the decode: more of them never pays
-        const int64_t items = tiles_n * ((m + mt - 1) / mt), rounds = (items + units - 1) / units;
+        const int64_t items = tiles_n * tm, rounds = (items + units - 1) / units;
         const double cost = (double)rounds * (stages * std::max(dec, 2.0 * mt) + 4000.0);
         if (!best || cost < 0.97 * best_cost) best = mt, best_cost = cost;
     }
     if (cost_out) *cost_out = best_cost;
     return best;
+}
+
+// The form of a dense launch: CTA pairs unless the one-CTA form is more than 2 % cheaper, and the rows per item
+struct KqForm {
+    bool pair;
+    int mt;
+};
+KqForm kq_choose(int64_t n, int64_t m, int nb, int ksplit, int sms, int pairs) {
+    const double stages = 4.0 * nb / ksplit;
+    double c1 = 0.0, c2 = 0.0;
+    const int mt1 = kq_rows_per_item(m, (n + 127) / 128 * ksplit, sms, stages, 300.0, &c1);
+    const int mt2 = pairs > 0 ? kq_rows_per_item(m, (n + 255) / 256 * ksplit, pairs, stages, 300.0, &c2) : 0;
+    if (pairs > 0 && c2 <= 1.02 * c1) return {true, mt2};
+    return {false, mt1};
 }
 
 }  // namespace
@@ -1112,17 +1126,9 @@ static int kq_dense(int fmt, const void* t16, int64_t n, int64_t k, const void* 
     const int sms = kq_sms();
     if (msub == 0)
         if (int rc = kq_configure<true>(fmt, &pairs)) return rc;
-    const double stages = 4.0 * p.nb / ksplit;
-    bool pair = false;
-    if (msub) {
-        p.mt = 128 * msub;
-    } else {
-        double c1 = 0.0, c2 = 0.0;
-        const int mt1 = kq_rows_per_item(m, (n + 127) / 128 * ksplit, sms, stages, 300.0, &c1);
-        const int mt2 = pairs > 0 ? kq_rows_per_item(m, (n + 255) / 256 * ksplit, pairs, stages, 300.0, &c2) : 0;
-        pair = pairs > 0 && c2 <= 1.02 * c1;
-        p.mt = pair ? mt2 : mt1;
-    }
+    const KqForm form = msub ? KqForm{false, 128 * msub} : kq_choose(n, m, p.nb, ksplit, sms, pairs);
+    const bool pair = form.pair;
+    p.mt = form.mt;
     CUtensorMap ta;                                                                 // one box is 64 inputs of all the rows that a CTA loads for an item
     p.box_rows = (uint32_t)(pair ? p.mt / 2 : p.mt);
     if (int rc = kyb_make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a, (uint64_t)m, (uint64_t)k, (uint64_t)lda * 2, p.box_rows, 64)) return rc;
@@ -1137,6 +1143,7 @@ static int kq_dense(int fmt, const void* t16, int64_t n, int64_t k, const void* 
         if ((uintptr_t)d[i] & 15) p.tma_out = 0;
     for (int i = 0; i < nout && p.tma_out; ++i)
         if (int rc = kyb_make_tmap_2d(&outs.m[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, d[i], (uint64_t)m, (uint64_t)(col0 + n), (uint64_t)ldd * 2, 32, 64)) return rc;
+    KYB_REQUIRE((int64_t)p.tiles_n * p.tiles_m * ksplit < (1ll << 31), "m=%lld n=%lld: too many output tiles", (long long)m, (long long)n);
     const int items = p.tiles_n * p.tiles_m * ksplit;
     if (int rc = pair ? kq_launch<true>(fmt, ta, outs, p, items, pairs, (cudaStream_t)stream) : kq_launch<false>(fmt, ta, outs, p, items, sms, (cudaStream_t)stream)) return rc;
     if (ksplit == 1) return KYB_OK;
@@ -1153,6 +1160,18 @@ extern "C" int kyb_gemm_kq(int fmt, const void* t16, int64_t n, int64_t k, const
     KYB_REQUIRE(d && ((uintptr_t)d & 1) == 0, "null or odd output pointer");
     void* outs[1] = {d};
     return kq_dense(fmt, t16, n, k, a, lda, m, gscale, outs, 1, ldd, 0, msub, stream);
+}
+
+// Diagnostics: the form that kyb_gemm_kq (split = 1) or kyb_gemm_kq_splitk takes for a shape. out3 = {1 by CTA pairs / 0 one CTA, activation rows per item, items}.
+// Without a device: as on 148 SMs.
+extern "C" int kyb_gemm_kq_plan(int fmt, int64_t n, int64_t k, int64_t m, int split, int64_t* out3) {
+    KYB_REQUIRE(fmt >= 0 && fmt < KYB_FMT_COUNT && n > 0 && m > 0 && k > 0 && k % 256 == 0 && split >= 1 && split <= 8 && out3, "bad arguments");
+    int pairs = 0, dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || kq_configure<true>(fmt, &pairs) != KYB_OK) pairs = kq_sms() / 2;
+    (void)cudaGetLastError();
+    const KqForm f = kq_choose(n, m, (int)(k / 256), split, kq_sms(), pairs);
+    out3[0] = f.pair, out3[1] = f.mt, out3[2] = (f.pair ? (n + 255) / 256 : (n + 127) / 128) * ((m + f.mt - 1) / f.mt) * split;
+    return KYB_OK;
 }
 
 // Split-k for products with fewer output tiles than SMs (e.g. 2048 x 3072 outputs from 12288 inputs: 96 tiles of 256 x 256): the k-blocks are cut into `split`

@@ -382,6 +382,14 @@ def gemm_kq(fmt, t16: torch.Tensor, n: int, k: int, a: torch.Tensor, gscale: flo
     return d
 
 
+def gemm_kq_plan(fmt, n: int, k: int, m: int, split: int = 1) -> dict:
+    """The form gemm_kq takes for a shape: by CTA pairs or not, activation rows per work item, work items."""
+    import ctypes
+    out = (ctypes.c_int64 * 3)()
+    _lib.check(_lib.lib().kyb_gemm_kq_plan(_fmt(fmt), n, k, m, split, out))
+    return dict(pair=bool(out[0]), rows=out[1], items=out[2])
+
+
 def gemm_kq_ag(fmt, t16: torch.Tensor, n: int, k: int, a: torch.Tensor, peer_ptrs, ldd: int, col0: int, gscale: float = 1.0, msub: int = 0) -> None:
     """gemm_kq whose epilogue stores every tile into the [m, ldd] fp16 output matrix of every rank (peer_ptrs: peer-mapped base addresses, own rank included) at
     column col0: the all-gather of an N-sharded linear happens inside the GEMM. The caller synchronises the ranks around the call."""
