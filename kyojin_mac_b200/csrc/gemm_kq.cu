@@ -564,7 +564,8 @@ __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.
 __device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
-// a bounded wait of the whole warp whose answer is a vote, so that what depends on it stays uniform
+// A bounded wait of the whole warp whose answer is a vote. Every wait of this kernel is one: lanes poll on their own and may give up at different times, and behind
+// each wait stand warp-wide instructions (tcgen05.ld / st, __syncwarp) that must not be met by a part of the warp.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_fast(bar, parity)) != 0; }
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void epilogue_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }      // the four epilogue warps
@@ -762,7 +763,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_kq_kernel(const __grid_con
             const int nsub = it.nn > 128 ? 2 : 1;
             for (int sub = 0; sub < nsub; ++sub) {
                 const uint32_t slot = nsub == 2 ? (uint32_t)sub : next;
-                if (!failed && !mbar_wait_fast(accf0 + 8 * slot, (uses >> slot) & 1u)) failed = true;
+                if (!failed && !mbar_wait_warp(accf0 + 8 * slot, (uses >> slot) & 1u)) failed = true;
                 uses ^= 1u << slot, next = slot ^ 1u;
                 tc_fence_after();
                 const int cols = min(it.nn - 128 * sub, 128);
@@ -909,7 +910,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_kq_kernel(const __grid_con
             kq_refill<FMT, 0>(wk.ptr, lane, tr);
 #define KYB_KQ_WAIT(H)                                                               \
     {                                                                                \
-        if (!mbar_wait_fast(empty + 8 * (H), parity)) failed = true;                 \
+        if (!mbar_wait_warp(empty + 8 * (H), parity)) failed = true;                 \
         tc_fence_after();                                                            \
     }
 #define KYB_KQ_PUBLISH(H)                                                            \
