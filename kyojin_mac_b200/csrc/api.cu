@@ -3,6 +3,7 @@
 #include <string.h>
 
 #include <mutex>
+#include <unordered_map>
 
 #include "kyb_common.cuh"
 
@@ -30,6 +31,21 @@ unsigned int* kyb_device_status_word() {
         g_status_words[dev] = (unsigned int*)p;
     }
     return g_status_words[dev];
+}
+
+int kyb_allow_smem(const void* kern) {
+    static std::mutex mu;
+    static std::unordered_map<const void*, uint64_t> done;             // bit d: set on device d
+    int dev = 0;
+    KYB_CUDA(cudaGetDevice(&dev));
+    KYB_REQUIRE(dev >= 0 && dev < 64, "device ordinal %d out of range", dev);
+    std::lock_guard<std::mutex> lk(mu);
+    uint64_t& mask = done[kern];
+    if (!(mask >> dev & 1)) {
+        KYB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));   // of 227 KB: leaves room for the few static words
+        mask |= 1ull << dev;
+    }
+    return KYB_OK;
 }
 
 extern "C" {

@@ -17,7 +17,6 @@
 #include <map>
 #include <mutex>
 #include <tuple>
-#include <unordered_map>
 
 #include "t16_decode.cuh"
 
@@ -1118,21 +1117,6 @@ GemvPlan make_plan(int fmt, int64_t n, int64_t k, int64_t m, bool sums = true) {
     return pl;
 }
 
-// opt in to large dynamic shared memory once per device and kernel (the attribute is per device and per function)
-int ensure_smem_attr(const void* kern) {
-    static std::mutex mu;
-    static std::unordered_map<const void*, unsigned> done;
-    int dev = 0;
-    KYB_CUDA(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lk(mu);
-    unsigned& mask = done[kern];
-    if (!(mask & (1u << (dev & 31)))) {
-        KYB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024 - 1024)));   // leaves room for the few static words
-        mask |= 1u << (dev & 31);
-    }
-    return KYB_OK;
-}
-
 // launches `kern` plainly or, when chained, with programmatic stream serialization (its CTAs may become resident while the preceding kernel of the stream drains)
 int launch_maybe_chained(const void* kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, void** args, bool chained, const char* what) {
     cudaLaunchConfig_t cfg = {};
@@ -1178,7 +1162,7 @@ int launch_gemv(int fmt, const GemvPlan& pl, const void* t16, int64_t n, int64_t
     p.partial_only = (staged || pl.local) ? 1 : 0, p.pdl = chained ? 1 : 0;
     p.local = (pl.local && !sums_only) ? 1 : 0;                    // chunk sums asked for by the caller go to its buffer as in form (b)
     const void* kern = gemv_kernel_ptr(fmt, variant_of(m));
-    if (int rc = ensure_smem_attr(kern)) return rc;
+    if (int rc = kyb_allow_smem(kern)) return rc;
     void* args[] = {(void*)&p};
     if (int rc = launch_maybe_chained(kern, dim3((unsigned)pl.grid), dim3((unsigned)pl.warps * 32), pl.smem, st, args, chained, "gemv_t16")) return rc;
     if (staged && !sums_only) {
@@ -1377,7 +1361,7 @@ extern "C" int kyb_gemv_group_t16(int fmt, const void* t16, const void* t16b, in
                        : fmt == KYB_FMT_Q2_K ? (const void*)kyb::gemv_group_kernel<KYB_FMT_Q2_K>
                        : fmt == KYB_FMT_IQ4_XS ? (const void*)kyb::gemv_group_kernel<KYB_FMT_IQ4_XS>
                                              : (const void*)kyb::gemv_group_kernel<KYB_FMT_NVFP4>;
-    if (int r = ensure_smem_attr(kern)) return r;
+    if (int r = kyb_allow_smem(kern)) return r;
     void* args[] = {(void*)&p};
     KYB_CUDA(cudaLaunchKernel(kern, dim3((unsigned)sms), dim3((unsigned)warps * 32), args, smem + 64, (cudaStream_t)stream));
     return KYB_OK;

@@ -10,6 +10,8 @@
 
 // ------------------------------------------------------------------------------------------------ host side
 void kyb_set_error(const char* fmt, ...);
+// opts a kernel in to large dynamic shared memory (up to 226 KB), once per device: the attribute belongs to the kernel on one device, not to the process
+int kyb_allow_smem(const void* kern);
 unsigned int* kyb_device_status_word();   // per-device word in global memory, zero-initialised (nullptr on failure)
 // grouped products: zero the output rows of the sorted positions [*first, s) (slots that belong to no expert segment); first = device pointer to off[E]
 int kyb_zero_tail_rows(void* d, int64_t ldd, int64_t n, const void* row_map, const void* first, int64_t s, cudaStream_t st);

@@ -580,11 +580,8 @@ extern "C" int kyb_moe_plan(const void* ids, const void* wts, const void* rank, 
     KYB_REQUIRE(ids, "null pointer");
     KYB_REQUIRE(E > 0 && E <= 8192 && P > 0 && P < (1ll << 31) && topk > 0 && mt > 0, "E=%d P=%lld topk=%d mt=%d out of range", E, (long long)P, topk, mt);
     const size_t smem = (size_t)(2 * (E + 1) + 33) * sizeof(uint32_t);
-    static bool configured = false;
-    if (!configured && smem > 48 * 1024) {
-        KYB_CUDA(cudaFuncSetAttribute(kyb::moe_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((2 * 8193 + 33) * sizeof(uint32_t))));
-        configured = true;
-    }
+    if (smem > 48 * 1024)
+        if (int rc = kyb_allow_smem((const void*)kyb::moe_plan_kernel)) return rc;
     const unsigned ctas = P >= 4096 ? 8u : 1u;                                  // one cluster; 8 is the portable cluster size
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas), cfg.blockDim = dim3(kyb::PLAN_THREADS), cfg.dynamicSmemBytes = smem, cfg.stream = (cudaStream_t)stream;
@@ -656,35 +653,6 @@ extern "C" int kyb_moe_combine(const void* y, int64_t ldy, const void* scs, cons
     return kyb_launch_check("moe_combine");
 }
 
-template <typename XT, int TT>
-static int launch_router(const void* x, int64_t ldx, const float* gw, const float* sgw, int64_t T, int E, int64_t H, float* lg, int64_t ldl, cudaStream_t st) {
-    const size_t smem = (size_t)TT * (size_t)H * sizeof(XT);
-    static bool configured = false;                                         // one flag per instantiation (a template static)
-    if (!configured) {
-        KYB_CUDA(cudaFuncSetAttribute(kyb::router_logits_kernel<XT, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        configured = true;
-    }
-    const int64_t gx = (T + TT - 1) / TT;
-    const int R = E + (sgw ? 1 : 0);
-    if (T <= 128) {
-        // few tokens (at 300 the other kernel, which reads a weight row for four rows' worth of staged tokens, is faster: 62 us against 104): the weight rows are dealt two by two to the warps of as many CTAs as there are SMs (4 warps per CTA while that still leaves SMs without one)
-        static bool few_configured = false;
-        if (!few_configured) {
-            KYB_CUDA(cudaFuncSetAttribute(kyb::router_logits_few_kernel<XT, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-            few_configured = true;
-        }
-        const int warps = gx * ((R + 15) / 16) <= 74 ? 4 : 8;
-        const int64_t gy = std::min<int64_t>((R + 2 * warps - 1) / (2 * warps), std::max<int64_t>(1, (148 + gx / 2) / gx));
-        kyb::router_logits_few_kernel<XT, TT><<<dim3((unsigned)gx, (unsigned)gy), warps * 32, smem, st>>>((const XT*)x, ldx, gw, sgw, (int)T, E, (int)H, lg, ldl);
-        return kyb_launch_check("router_logits_few");
-    }
-    const int threads = T >= 1024 ? 512 : 256;                               // many tokens: 16 warps per CTA hide the L2 latency of the weight rows
-    const int ymax = (R + threads / 8 - 1) / (threads / 8);   // warps x 4 rows per pass
-    const int gy = (int)std::min<int64_t>(ymax, std::max<int64_t>(1, (2 * 148 + gx - 1) / gx));   // few tokens: spread the weight rows over more CTAs
-    kyb::router_logits_kernel<XT, TT><<<dim3((unsigned)gx, (unsigned)gy), threads, smem, st>>>((const XT*)x, ldx, gw, sgw, (int)T, E, (int)H, lg, ldl);
-    return kyb_launch_check("router_logits");
-}
-
 static int router_sms() {
     static int sms = 0;
     if (!sms) {
@@ -695,14 +663,32 @@ static int router_sms() {
     return sms;
 }
 
+template <typename XT, int TT>
+static int launch_router(const void* x, int64_t ldx, const float* gw, const float* sgw, int64_t T, int E, int64_t H, float* lg, int64_t ldl, cudaStream_t st) {
+    const size_t smem = (size_t)TT * (size_t)H * sizeof(XT);
+    const int64_t gx = (T + TT - 1) / TT;
+    const int R = E + (sgw ? 1 : 0), sms = router_sms();
+    if (T <= 128) {
+        // few tokens (at 300 the other kernel, which reads a weight row for four rows' worth of staged tokens, is faster: 62 us against 104): the weight rows are
+        // dealt two by two to the warps of as many CTAs as there are SMs (4 warps per CTA while that still leaves SMs without one)
+        if (int rc = kyb_allow_smem((const void*)kyb::router_logits_few_kernel<XT, TT>)) return rc;
+        const int warps = gx * ((R + 15) / 16) <= sms / 2 ? 4 : 8;
+        const int64_t gy = std::min<int64_t>((R + 2 * warps - 1) / (2 * warps), std::max<int64_t>(1, (sms + gx / 2) / gx));
+        kyb::router_logits_few_kernel<XT, TT><<<dim3((unsigned)gx, (unsigned)gy), warps * 32, smem, st>>>((const XT*)x, ldx, gw, sgw, (int)T, E, (int)H, lg, ldl);
+        return kyb_launch_check("router_logits_few");
+    }
+    if (int rc = kyb_allow_smem((const void*)kyb::router_logits_kernel<XT, TT>)) return rc;
+    const int threads = T >= 1024 ? 512 : 256;                               // many tokens: 16 warps per CTA hide the L2 latency of the weight rows
+    const int ymax = (R + threads / 8 - 1) / (threads / 8);   // warps x 4 rows per pass
+    const int gy = (int)std::min<int64_t>(ymax, std::max<int64_t>(1, (2 * sms + gx - 1) / gx));   // few tokens: spread the weight rows over more CTAs
+    kyb::router_logits_kernel<XT, TT><<<dim3((unsigned)gx, (unsigned)gy), threads, smem, st>>>((const XT*)x, ldx, gw, sgw, (int)T, E, (int)H, lg, ldl);
+    return kyb_launch_check("router_logits");
+}
+
 template <typename XT, int WR, int RE, int THREADS>
 static int launch_router_wres(const void* x, int64_t ldx, const float* gw, const float* sgw, int64_t T, int E, int64_t H, float* lg, int64_t ldl, cudaStream_t st) {
     const size_t smem = (size_t)WR * (size_t)H * sizeof(float);
-    static bool configured = false;
-    if (!configured) {
-        KYB_CUDA(cudaFuncSetAttribute(kyb::router_logits_wres_kernel<XT, WR, RE, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        configured = true;
-    }
+    if (int rc = kyb_allow_smem((const void*)kyb::router_logits_wres_kernel<XT, WR, RE, THREADS>)) return rc;
     const int R = E + (sgw ? 1 : 0), gx = (R + WR - 1) / WR;
     const int64_t per_pass = (int64_t)(THREADS / 32) * RE;
     const int gy = (int)std::max<int64_t>(1, std::min<int64_t>((T + per_pass - 1) / per_pass, router_sms() / gx));   // one wave of CTAs, one CTA per SM
