@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(512) router_logits_kernel(const XT* __restrict
 }
 
 // The same for few tokens (decode), where the walk along a weight row is one load latency after the other: two rows per warp instead of four spread the rows over
-// twice the warps, and the weights of the next D steps are in flight while D steps are summed (one step at a time: 55 us for 64 tokens, 257 x 7168; now 13 us).
+// twice the warps, and the weights of the next D steps are in flight while D steps are summed (64 tokens, 257 x 7168, gate in HBM: 48 us one step at a time, 17 us so).
 // The sums are formed in the same order.
 template <typename XT, int TT>
 __global__ void __launch_bounds__(256) router_logits_few_kernel(const XT* __restrict__ x, int64_t ldx, const float* __restrict__ gw, const float* __restrict__ sgw, int T, int E, int H,
@@ -663,18 +663,41 @@ static int router_sms() {
     return sms;
 }
 
+// The few-token kernel: gx CTAs along the tokens, gy along the weight rows, two rows per warp and pass.
+struct RouterFew {
+    int warps;
+    int64_t gy, passes;
+};
+static RouterFew router_few(int64_t gx, int R, int sms) {
+    RouterFew f;
+    f.warps = gx * ((R + 15) / 16) <= sms / 2 ? 4 : 8;                        // 4 warps per CTA while that still leaves SMs without one
+    f.gy = std::min<int64_t>((R + 2 * f.warps - 1) / (2 * f.warps), std::max<int64_t>(1, (sms + gx / 2) / gx));
+    f.passes = (R + f.gy * f.warps * 2 - 1) / (f.gy * f.warps * 2);
+    return f;
+}
+// Few tokens: which of the two kernels. The few-token kernel's time is its passes over the weight rows times a pass along a row (8.5 us at 3072 inputs, 15.5 at 7168);
+// the other one walks a row one load latency after the other (21 us at 3072, 48 at 7168 with the gate in HBM) but covers four rows of a staged token read, so it
+// hardly grows up to 128 tokens. Measured, the other kernel against this one, gate in HBM: one pass, 64 x 2048 inputs 9.6 / 7.0 us, 256 x 7168 48 / 15.6; two,
+// 256 x 2048 (L2) 10.0 / 14.4, 256 x 3072 20 / 18, 256 x 7168 48 / 31; three, 512 x 4096 28.6 / 30, 384 x 5120 35 / 31.8; four, 512 x 4096 29.6 / 39, 256 x 16384
+// 121 / 113. Short rows leave half of its eight steps empty: eight tokens, 256 x 512 4.4 / 5.2 us, 8 x 1024 4.9 / 5.5 but 64 x 1024 5.9 / 5.6 (while four warps
+// per CTA suffice: 256 x 1024, 64 tokens 6.2 / 6.7).
+static bool router_takes_few(const RouterFew& f, int64_t T, int tt, int R, int64_t H) {
+    if (T > 128 || f.passes > 4) return false;
+    static const int64_t from[5] = {0, 2048, 3072, 5120, 12288};             // inputs from which this many passes are the faster way
+    if (H >= from[f.passes]) return true;
+    if (f.passes > 1) return false;
+    return H >= 1024 ? tt < 8 || (R >= 16 && f.warps == 4) : T <= 4;
+}
+
 template <typename XT, int TT>
 static int launch_router(const void* x, int64_t ldx, const float* gw, const float* sgw, int64_t T, int E, int64_t H, float* lg, int64_t ldl, cudaStream_t st) {
     const size_t smem = (size_t)TT * (size_t)H * sizeof(XT);
     const int64_t gx = (T + TT - 1) / TT;
     const int R = E + (sgw ? 1 : 0), sms = router_sms();
-    if (T <= 128) {
-        // few tokens (at 300 the other kernel, which reads a weight row for four rows' worth of staged tokens, is faster: 62 us against 104): the weight rows are
-        // dealt two by two to the warps of as many CTAs as there are SMs (4 warps per CTA while that still leaves SMs without one)
+    const RouterFew few = router_few(gx, R, sms);
+    if (router_takes_few(few, T, TT, R, H)) {
         if (int rc = kyb_allow_smem((const void*)kyb::router_logits_few_kernel<XT, TT>)) return rc;
-        const int warps = gx * ((R + 15) / 16) <= sms / 2 ? 4 : 8;
-        const int64_t gy = std::min<int64_t>((R + 2 * warps - 1) / (2 * warps), std::max<int64_t>(1, (sms + gx / 2) / gx));
-        kyb::router_logits_few_kernel<XT, TT><<<dim3((unsigned)gx, (unsigned)gy), warps * 32, smem, st>>>((const XT*)x, ldx, gw, sgw, (int)T, E, (int)H, lg, ldl);
+        kyb::router_logits_few_kernel<XT, TT><<<dim3((unsigned)gx, (unsigned)few.gy), few.warps * 32, smem, st>>>((const XT*)x, ldx, gw, sgw, (int)T, E, (int)H, lg, ldl);
         return kyb_launch_check("router_logits_few");
     }
     if (int rc = kyb_allow_smem((const void*)kyb::router_logits_kernel<XT, TT>)) return rc;
