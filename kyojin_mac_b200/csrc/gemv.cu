@@ -1034,72 +1034,99 @@ int canonical_chunk(int ntiles, int nb) {
     return best;
 }
 
-// Warps per CTA, k-parts and the way work is dealt: the launch that a small cost model (microseconds) finds cheapest.
-//   stream   the tiles at 5.6 TB/s or at the issue rate of a tile (about 115 / 220 / 310 / 400 clocks of an SM for one to four column tiles), divided by how even the
-//            shares of the warps are (whole row tiles: form (a), one k-part; runs of chunks: form (b); the square root, because the other warps of an SM run faster
-//            when one has finished) and of the CTAs (whole row tiles per CTA: form (c)), by the share of SMs in use and by an occupancy factor: 12 warps (three
-//            per scheduler) measured best for up to 16 rows, 14 and 16 lose 8-10 % again, 10 and fewer lose to latency
-//   staging  every CTA stages the activations of its k-part before its first tile: 0.022 us per 256 inputs and row measured, 0.085 us with the gated activation
-//            formed on the way (the plan does not know which, 0.027 is taken). So form (b) cuts k into as many parts as leave the SMs evenly used: Q6_K 5120 x 27648,
-//            eight rows, 3 parts of 36 blocks and 10 warps -> 18 parts of 6 blocks and 12 warps: 38.1 -> 30.3 us, gated 59.3 -> 33.0 us; one row 31.4 -> 27.3, gated
-//            38.9 -> 30.0 us
-//   finish   form (b): the chunk sums through the workspace (written and read at 4 TB/s) and about 3.5 us for the finalize launch inside a chain
+// Warps per CTA, k-parts and the way work is dealt: the launch that a small cost model (microseconds) finds cheapest. Fitted to 6400 timings of chained launches (770
+// shapes from 16 x 256 to 65536 x 28672, every format, 1 to 32 rows, plain and gated, every form and warp counts 4 to 12); what it picks is on average 2 % slower
+// than the best of the forms tried on a shape.
+//   stream   the tiles at 6.2 TB/s or at the issue rate of a tile (133 / 206 / 330 / 282 clocks of an SM for one to four column tiles), divided by how even the shares
+//            of the warps are (whole row tiles: form (a), one k-part; runs of chunks: form (b); the square root, because the other warps of an SM run faster when
+//            one has finished) and of the CTAs (whole row tiles per CTA: form (c)), by the share of SMs in use and by the occupancy: 12 warps (three per scheduler)
+//            measured best, 8 (two) next; uneven counts per scheduler are worse than either, 14 and 16 lose 8-10 % again
+//   serial   a warp works through its tiles one after the other, 0.6 to 1.8 us each, however empty the SM is: what few tiles there are is cut finely. NVFP4
+//            320 x 1792, three rows, one warp per row tile 6.2 us, form (c) 2.8. It overlaps the stream only in part: both enter with an exponent
+//   staging  every CTA stages the activations of its k-part before its first tile: 1.2 us per round of four items (32 inputs of a row) and thread, 0.024 us per 256
+//            inputs and row (between plain and gated rows, the plan does not know which). Form (b) cuts k into as many parts as leave the SMs evenly used: Q6_K
+//            5120 x 27648, eight rows, 3 parts of 36 blocks and 10 warps -> 18 parts of 6 blocks and 12 warps: 38.1 -> 30.3 us, gated 59.3 -> 33.0 us
+//   finish   form (b): the chunk sums through the workspace (written and read at 4.8 TB/s), 1.2 us for the finalize launch inside a chain and 0.12 us per chunk; 0.46 us
+//            more where the finalize kernel finds no registers beside the product's CTAs, so that its launch can't overlap them (1024 x 1792, 20 rows, 12 warps 7.6 us,
+//            8 warps 5.3)
+//   overlap  in a chain the CTAs of the next launch start their copies beside this one's if both fit an SM: 0.3 us off a launch of form (a) or (c) (more CTAs: more of
+//            it), less where a warp of form (a) walks long
 // sums: chunk sums may go through a workspace; without, only form (a) over one k-part and form (c) are left (no warps in the plan: neither fits).
 GemvPlan search_plan(int fmt, int64_t n, int64_t k, int64_t m, bool sums) {
     const int sms = device_sms();
     const int nb = (int)(k / 256), ntiles = (int)((n + 15) / 16);
-    const size_t smem_cap = 226 * 1024;
+    const size_t smem_cap = 226 * 1024, smem_sm = 228 * 1024;
     const int kc = canonical_chunk(ntiles, nb), nchunks = (nb + kc - 1) / kc;
     const int v = variant_of(m), nt = VAR_NT[v], mst = VAR_MST[v];
     const int max_warps = std::min(12, kyb::gemv_threads(fmt, nt) / 32);
-    const double tiles = (double)ntiles * nb, tile_clk = nt == 1 ? 115.0 : nt == 2 ? 220.0 : nt == 3 ? 310.0 : 400.0;
-    const double stream_us = std::max(tiles * (double)kyb_tile_bytes(fmt) / 5.6e6, tiles * tile_clk / sms / 1900.0);
-    static const double OCC[13] = {0.0, 0.3, 0.4, 0.5, 0.60, 0.62, 0.68, 0.74, 0.82, 0.84, 0.90, 0.93, 1.0};
+    const int regs = nt <= 2 ? 128 : max_warps == 8 ? 250 : 168, finalize_regs = 16384;   // a thread's; what the finalize kernel's CTAs want of an SM's 65536
+    const double tiles = (double)ntiles * nb, tile_clk = nt == 1 ? 133.0 : nt == 2 ? 206.0 : nt == 3 ? 330.0 : 282.0;
+    const double stream_us = std::max(tiles * (double)kyb_tile_bytes(fmt) / 6.2e6, tiles * tile_clk / sms / 1900.0);
+    const double tile_us = nt == 1 ? 0.61 : nt == 2 ? 0.80 : nt == 3 ? 0.98 : 1.81;
+    static const double OCC[13] = {0.0, 0.0, 0.0, 0.0, 0.71, 0.0, 0.49, 0.0, 0.76, 0.0, 0.635, 0.0, 1.0};
     auto occupancy = [&](int warps) { return max_warps == 8 ? std::min(1.0, 0.52 + 0.06 * warps) : OCC[warps]; };
-    auto staging_us = [&](int blocks) { return 0.027 * blocks * (double)m; };
-    // a warp works through its tiles one after the other: about 0.42 us per tile even when the SM is nearly empty (more with more column tiles)
-    auto serial_us = [&](double rounds, int tiles_each) { return rounds * tiles_each * (nt == 1 ? 0.42 : nt == 2 ? 0.55 : nt == 3 ? 0.72 : 0.9); };
-    const double finish_us = 3.5 + (double)nchunks * (double)m * (double)n * 8.0 / 4.0e6;
-    GemvPlan best{};
-    double best_us = 0.0;
+    auto busy_us = [&](double stream, double walk) { return std::pow(std::pow(stream, 2.27) + std::pow(walk * tile_us, 2.27), 1.0 / 2.27); };
+    auto staging_us = [&](int blocks, int warps) { return 1.21 * blocks * 8.0 * nt * mst / (4.0 * 32.0 * warps) + 0.0237 * blocks * (double)m; };
+    auto overlap = [&](int warps, size_t smem) {
+        const int fit = std::min(65536 / (32 * warps * regs), (int)(smem_sm / (smem + 1024)));
+        return fit < 2 ? 0.0 : fit < 3 ? 1.0 : 1.4;
+    };
+    const double finish_us = 1.22 + (double)nchunks * (double)m * (double)n * 8.0 / 4.8e6 + 0.125 * nchunks;
+    GemvPlan best{}, rows{};
+    double best_us = 0.0, rows_us = 0.0, rows_rank = 0.0;
+    auto offer = [&](double us, const GemvPlan& pl) {
+        if (best.warps == 0 || us < best_us) best_us = us, best = pl;
+    };
     for (int ksplit = 1; ksplit <= std::min(nchunks, sms); ++ksplit) {
         const int cpp = (nchunks + ksplit - 1) / ksplit;
         if ((nchunks + cpp - 1) / cpp != ksplit) continue;               // one representative per distinct split
         const int kbp = std::min(nb, cpp * kc), grid = sms / ksplit * ksplit;
-        for (int warps = 4; warps <= max_warps; ++warps) {
+        for (int warps = 4; warps <= max_warps; warps += 2) {
             const size_t smem = plan_smem(fmt, nt, mst, kbp, warps, kyb::GEMV_DSTAGES);
             if (smem > smem_cap) continue;
-            const double wp = (double)(grid / ksplit) * warps;                                  // warps of a part
+            const double wp = (double)(grid / ksplit) * warps, both = overlap(warps, smem);     // warps of a part
             const double parts = (double)nchunks / ((double)ksplit * cpp);                      // the last part may be shorter
             const double common = parts * ((double)grid / sms) * occupancy(warps);
             for (int aligned = 0; aligned < 2; ++aligned) {
-                if (!(aligned && ksplit == 1) && !sums) continue;
+                const bool one_step = aligned && ksplit == 1;
+                if (!one_step && !sums) continue;
                 const double upw = aligned ? ntiles / wp : (double)ntiles * cpp / wp;           // row tiles or units per warp
-                const double balance = std::sqrt(upw / std::ceil(upw));
-                const double us = std::max(stream_us / (balance * common), serial_us(std::ceil(upw), aligned ? kbp : kc)) + staging_us(kbp) + (aligned && ksplit == 1 ? 0.0 : finish_us);
-                if (best.warps == 0 || us < best_us) best_us = us, best = GemvPlan{nt, mst, warps, kyb::GEMV_DSTAGES, kbp, ksplit, grid, smem, kc, nchunks, cpp, aligned, 0};
+                const double share = upw / std::ceil(upw), walk = std::ceil(upw) * (aligned ? kbp : kc);
+                const GemvPlan pl{nt, mst, warps, kyb::GEMV_DSTAGES, kbp, ksplit, grid, smem, kc, nchunks, cpp, aligned, 0};
+                const double us = busy_us(stream_us / (std::sqrt(share) * common), walk) + staging_us(kbp, warps);
+                if (one_step) {
+                    // Form (a), the number of warps: where a warp has one or two row tiles, those with fewer leave nothing for the others to run faster on, so even
+                    // shares count in full (NVFP4 18062 x 3072, one row, 12 warps for 0.6 row tiles each 13.2 us, 8 warps 10.3).
+                    const double extra = both * (0.0244 * walk - 0.302), rank = us + extra + (upw <= 2.0 && nb >= 4 ? stream_us / common * (1.0 / share - 1.0 / std::sqrt(share)) : 0.0);
+                    if (rows.warps == 0 || rank < rows_rank) rows_rank = rank, rows_us = us + extra, rows = pl;
+                } else {
+                    offer(us + finish_us + (65536 - 32 * warps * regs < finalize_regs ? 0.46 : 0.0), pl);
+                }
             }
         }
     }
+    if (rows.warps > 0) offer(rows_us, rows);
     // Form (c): CTA c owns whole row tiles (the product runs as long as the CTA with the most), the whole of k is staged in every CTA, so up to 8 activation rows and
-    // only while that fits shared memory; at least 64 CTAs must get work. It needs no second launch: taken instead of form (b) while the uneven shares of the CTAs
-    // cost less than 2.5 us (4096 x 4096, one row 7.4 -> 5.2 us, with the warp count that deals the chunks evenly 4.3 us; 10240 x 5120 10.2 -> 9.6; 5120 x 8192
-    // 9.3 -> 9.1), and instead of form (a) where the model says so.
-    if ((best.warps > 0 || !sums) && ntiles >= 64 && m <= 8) {
+    // only while that fits shared memory. It needs no second launch: with at least 64 CTAs at work it is taken instead of form (b) while the uneven shares of the CTAs
+    // cost less than 2.5 us (4096 x 4096, one row 7.4 -> 4.5 us, eight rows 13.3 -> 7.9; 5120 x 8192, eight rows 15.2 -> 13.9), else where the model says so. With fewer
+    // than 64 CTAs the staging is too long for many blocks and rows, most of all of gated rows: 256 x 2304, four rows 3.9 (b) / 3.1 us, 16 x 1792, eight gated rows
+    // 6.2 / 8.6.
+    if (m <= 8 && (ntiles >= 64 || nb * m <= 36)) {
         const int grid = std::min(sms, ntiles), rpc = (ntiles + grid - 1) / grid;
         const size_t cpart = (size_t)rpc * nchunks * (size_t)m * 16 * sizeof(float);
-        const double even = (double)ntiles / ((double)rpc * grid), t_us = tiles * (double)kyb_tile_bytes(fmt) / 5.0e6;
-        const bool few = !(best.aligned && best.ksplit == 1) && t_us * (1.0 / even - 1.0) < 2.5;
+        const double even = (double)ntiles / ((double)rpc * grid);
         GemvPlan c{};
         double c_us = 0.0;
-        for (int warps = max_warps; warps >= 8; --warps) {
+        for (int warps = 8; warps <= max_warps; warps += 2) {
             const size_t smem = plan_smem(fmt, nt, mst, nb, warps, kyb::GEMV_DSTAGES) + cpart;
             if (smem > smem_cap) continue;
-            const double upw = (double)rpc * nchunks / warps, balance = even * std::sqrt(upw / std::ceil(upw));
-            const double us = std::max(stream_us / (balance * ((double)grid / sms) * occupancy(warps)), serial_us(std::ceil(upw), kc)) + staging_us(nb);
+            const double upw = (double)rpc * nchunks / warps, balance = even * std::sqrt(upw / std::ceil(upw)), sum_rounds = std::ceil(rpc * 16.0 * m / (32.0 * warps));
+            const double us = busy_us(stream_us / (balance * ((double)grid / sms) * occupancy(warps)), std::ceil(upw) * kc) + staging_us(nb, warps) + 0.10 +
+                              0.0027 * sum_rounds * nchunks - 0.269 * overlap(warps, smem);
             if (c.warps == 0 || us < c_us) c_us = us, c = GemvPlan{nt, mst, warps, kyb::GEMV_DSTAGES, nb, 1, grid, smem, kc, nchunks, nchunks, 0, 1};
         }
-        if (c.warps > 0 && (few || c_us < best_us)) return c;
+        const bool one_launch = best.aligned && best.ksplit == 1, few = ntiles >= 64 && !one_launch && tiles * (double)kyb_tile_bytes(fmt) / 5.0e6 * (1.0 / even - 1.0) < 2.5;
+        if (c.warps > 0 && (few || best.warps == 0 || c_us < (one_launch ? 0.88 : 1.0) * best_us)) return c;   // from form (a) for a clear gain only
     }
     return best;
 }

@@ -26,7 +26,8 @@ def test_plans_are_runnable(fmt):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("fmt,n,k", [("q6_k", 1577, 6912), ("q4_k", 609, 5120), ("q5_k", 4100, 8192), ("q3_k", 865, 5888), ("nvfp4", 2400, 1280), ("q8_0", 33, 13568)])
+@pytest.mark.parametrize("fmt,n,k", [("q6_k", 1577, 6912), ("q4_k", 609, 5120), ("q5_k", 4100, 8192), ("q3_k", 865, 5888), ("nvfp4", 2400, 1280), ("q8_0", 33, 13568),
+                                     ("iq4_xs", 16, 1792), ("nvfp4", 320, 1792), ("q2_k", 5376, 512), ("q4_k", 38, 256)])
 def test_rows_do_not_depend_on_the_plan(fmt, n, k):
     from kyojin_mac_b200 import mma_gemv
     from kyojin_mac_b200.foreign_linear import DevPack
