@@ -12,7 +12,7 @@
 //   warp 0      TMA: activation boxes (64 rows x 64 inputs) into a ring of shared-memory stages
 //   warp 1      tcgen05.mma issuer (M = 128 output rows, A from tensor memory, two accumulator slots of 128 columns), tcgen05.commit hands stages back
 //   warps 2-5   epilogue: tcgen05.ld 16x256b, output scale, stmatrix.trans turns the fragments around into [activation row][output] staging tiles, which leave as
-//               tiled bulk stores or as coalesced row pieces
+//               tiled bulk stores (two warps per store of 32 rows x 64 outputs) or as coalesced row pieces
 //   warps 6-21  decoders: warp (q = warp % 4, j) owns row tile 2 q + (j & 1) of the CTA's 128 output rows (the tensor-memory lanes a warp may touch are those of its
 //               quarter q) and every second T16 tile of it (parity j >> 1). It keeps one T16 tile in registers, each unit refilled from its next tile right after its
 //               use (across items too), unpacks a 64-input quarter with LOP3 / PRMT into fp16 pairs, applies the block scales with half2 arithmetic (scale and
@@ -568,6 +568,7 @@ __device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uin
 // each wait stand warp-wide instructions (tcgen05.ld / st, __syncwarp) that must not be met by a part of the warp.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_fast(bar, parity)) != 0; }
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void half_barrier(int h) { asm volatile("bar.sync %0, 64;" ::"r"(2 + h) : "memory"); }   // the two epilogue warps of 64 outputs
 __device__ __forceinline__ void epilogue_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }      // the four epilogue warps
 __device__ __forceinline__ uint32_t pack_sat(uint32_t a, uint32_t b, float s) {
     __half2 h = sat_half2(__uint_as_float(a) * s, __uint_as_float(b) * s);
@@ -754,6 +755,8 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_kq_kernel(const __grid_con
     } else if (warp < 6) {
         // ---- epilogue: warp w may touch TMEM lanes [32 (w % 4), 32 (w % 4) + 32) = outputs n0 + 32 q ..
         const int q = warp & 3;
+        const bool issuer = elect_one() && (q & 1) == 0;                              // of the tiled stores of 64 outputs
+        const uint32_t xq = __reduce_max_sync(0xffffffffu, 32u * (uint32_t)(q & 2));  // first of the 64 outputs that this warp's half tile holds
         const uint32_t acce = PAIR ? map_to_rank(acce0, 0) : acce0;
         const uint32_t tq = tmem_base + ((uint32_t)(q * 32) << 16);
         uint32_t next = 0, uses = 0, ch = 0;                                          // accumulator slots as the MMA issuer deals them; staged 32-row chunks so far
@@ -767,6 +770,45 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_kq_kernel(const __grid_con
                 uses ^= 1u << slot, next = slot ^ 1u;
                 tc_fence_after();
                 const int cols = min(it.nn - 128 * sub, 128);
+                if (p.tma_out) {
+                    // ---- dense form with tiled bulk stores: 32 rows x 64 outputs per store. The two warps of 64 outputs share a half tile and a store, so no warp
+                    // waits for all four and two lanes issue the boxes; their operands are in uniform registers, the loop has no other form's branches.
+                    int row0 = it.m0 + 128 * sub;
+                    uint32_t ta = tq + slot * 128u;
+                    const bool mine = !failed && it.n0 + (int)xq < p.n;
+                    for (int left = cols; left > 0; left -= 32, ta += 32u, row0 += 32, ++ch) {
+                        uint32_t va[16], vb[16];                                        // outputs 32 q + g, + 8 and 32 q + 16 + g, + 8, activation rows 8 i + 2 t, + 1
+                        tmem_ld_16x256b_x4(ta, va);
+                        tmem_ld_16x256b_x4(ta + (16u << 16), vb);
+                        tmem_ld_wait();
+                        if (left <= 32) {                                               // this warp has read its quarter of the accumulator
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) {
+                                if constexpr (PAIR) mbar_arrive_remote(acce + 8 * slot);
+                                else mbar_arrive_a(acce + 8 * slot);
+                            }
+                        }
+                        const uint32_t stg = stg0 + (ch & 1u) * KQ_STG + 64u * xq;      // this half: 32 rows of 128 bytes
+                        const uint32_t c16 = 4u * (q & 1) + (lane >> 3), dst = stg + ((c16 ^ (lane & 7)) << 4) + (lane & 7) * 128u;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)                                    // matrices: outputs 0-7, 8-15, 16-23, 24-31 of the warp, activation rows 8 i .. 8 i + 7
+                            stmatrix_x4_trans(dst + 1024u * i, pack_sat(va[4 * i], va[4 * i + 1], it.gscale), pack_sat(va[4 * i + 2], va[4 * i + 3], it.gscale),
+                                              pack_sat(vb[4 * i], vb[4 * i + 1], it.gscale), pack_sat(vb[4 * i + 2], vb[4 * i + 3], it.gscale));
+                        fence_proxy_async_smem();
+                        // the other staging tile is free for the next chunk once the store issued from it has read it: waited for before the barrier
+                        if (issuer) tma_store_wait_read();
+                        half_barrier(q >> 1);
+                        if (issuer) {
+                            if (mine && row0 < it.m_end) {
+                                tma_store_2d(&outs.m[0], stg, p.col0 + it.n0 + (int)xq, row0);
+                                for (int pr = 1; pr < p.nout; ++pr) tma_store_2d(&outs.m[pr], stg, p.col0 + it.n0 + (int)xq, row0);
+                            }
+                            tma_store_commit();
+                        }
+                    }
+                    continue;
+                }
                 for (int c = 0; c < cols; c += 32) {
                     const int row0 = it.m0 + 128 * sub + c;
                     const bool last = c + 32 >= cols;
@@ -779,7 +821,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_kq_kernel(const __grid_con
                             tc_fence_before();
                             __syncwarp();
                             if (lane == 0) {
-                                if constexpr (PAIR) mbar_arrive_cluster(acce + 8 * slot);
+                                if constexpr (PAIR) mbar_arrive_remote(acce + 8 * slot);
                                 else mbar_arrive_a(acce + 8 * slot);
                             }
                         }
@@ -791,14 +833,12 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_kq_kernel(const __grid_con
                     }
                     // rows of the staged chunk that this warp will store (row stores): 8 rows, 16 (gated pair: 8) lanes of 16 bytes each
                     uint32_t orow[4];
-                    if (!p.tma_out) {
-                        const int per = p.glu ? 4 : 2;                                  // rows per store instruction
+                    const int per = p.glu ? 4 : 2;                                      // rows per store instruction
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int row = row0 + 8 * q + per * i + (p.glu ? lane >> 3 : lane >> 4);
-                            orow[i] = (uint32_t)row;
-                            if (p.row_map && i < 8 / per && row < it.m_end) orow[i] = p.row_map[row];
-                        }
+                    for (int i = 0; i < 4; ++i) {
+                        const int row = row0 + 8 * q + per * i + (p.glu ? lane >> 3 : lane >> 4);
+                        orow[i] = (uint32_t)row;
+                        if (p.row_map && i < 8 / per && row < it.m_end) orow[i] = p.row_map[row];
                     }
                     uint32_t va[16], vb[16];                                            // outputs 32 q + g, + 8 and 32 q + 16 + g, + 8, activation rows 8 i + 2 t, + 1
                     tmem_ld_16x256b_x4(tq + slot * 128u + (uint32_t)c, va);
@@ -808,7 +848,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_kq_kernel(const __grid_con
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) {
-                            if constexpr (PAIR) mbar_arrive_cluster(acce + 8 * slot);
+                            if constexpr (PAIR) mbar_arrive_remote(acce + 8 * slot);
                             else mbar_arrive_a(acce + 8 * slot);
                         }
                     }
@@ -839,19 +879,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_kq_kernel(const __grid_con
                             stmatrix_x4_trans(half_tile + 1024u * i, pack_sat(va[4 * i], va[4 * i + 1], gscale), pack_sat(va[4 * i + 2], va[4 * i + 3], gscale),
                                               pack_sat(vb[4 * i], vb[4 * i + 1], gscale), pack_sat(vb[4 * i + 2], vb[4 * i + 3], gscale));
                     }
-                    if (p.tma_out) {
-                        fence_proxy_async_smem();
-                        // the other staging tile is free for the next chunk once the stores issued from it have read it: waited for before the barrier
-                        if (warp == 2 && lane == 0) tma_store_wait_read();
-                        epilogue_barrier();
-                        if (warp == 2 && lane == 0) {
-                            if (!failed && row0 < it.m_end)
-                                for (int pr = 0; pr < p.nout; ++pr)
-                                    for (int h = 0; h < 2; ++h)
-                                        if (it.n0 + 64 * h < p.n) tma_store_2d(&outs.m[pr], stg + 4096u * h, p.col0 + it.n0 + 64 * h, row0);
-                            tma_store_commit();
-                        }
-                    } else {
+                    {
                         epilogue_barrier();
                         if (p.glu) {
 #pragma unroll
@@ -951,7 +979,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_kq_kernel(const __grid_con
 #undef KYB_KQ_PUBLISH
         }
     }
-    if (warp == 2 && lane == 0 && p.tma_out) tma_store_wait_all();                      // the staging buffer must outlive its stores
+    if ((warp == 2 || warp == 4) && p.tma_out) tma_store_wait_all();                      // the staging buffer must outlive its stores
     if (failed) atomicExch(p.status, KYB_DEV_TIMEOUT_GEMM);
     tc_fence_before();
     if constexpr (PAIR) cluster_sync_all();                                            // neither CTA frees tensor memory or leaves while the other may still signal it
@@ -1071,36 +1099,47 @@ int kq_launch(int fmt, const CUtensorMap& ta, const KybOutMaps& outs, kyb::KqPar
     return kyb_launch_check("gemm_kq");
 }
 
-// Activation rows per item (a multiple of 32, at most 256) for `tiles_n` column tiles on `units` CTAs or pairs: the whole rounds of equal items that cost least. A
-// stage of an item costs its MMAs (2 clocks per row) but never less than the decode of its weights (`dec` clocks), an item about 12 stages' worth of start and end.
-// The candidates are the item sizes, not the numbers of items, so any m has the same few of them and the widest one always counts.
-int kq_rows_per_item(int64_t m, int64_t tiles_n, int units, double stages, double dec, double* cost_out) {
-    int best = 0;
-    double best_cost = 0.0;
-    for (int mt = 256; mt >= 32; mt -= 32) {
-        const int64_t tm = (m + mt - 1) / mt;
-        if ((m + tm * 32 - 1) / (tm * 32) * 32 != mt) continue;                        // as many items of fewer rows cover m: that size is the candidate
-        if (mt < 96 && best) break;                                                    // narrower items are bound by the decode: more of them never pays
-        const int64_t items = tiles_n * tm, rounds = (items + units - 1) / units;
-        const double cost = (double)rounds * (stages * std::max(dec, 2.0 * mt) + 4000.0);
-        if (!best || cost < 0.97 * best_cost) best = mt, best_cost = cost;
-    }
-    if (cost_out) *cost_out = best_cost;
-    return best;
-}
-
-// The form of a dense launch: CTA pairs unless the one-CTA form is more than 2 % cheaper, and the rows per item
+// The form of a dense launch: CTA pairs or not, and activation rows per item (a multiple of 32, at most 256): what a cost model in clocks finds cheapest. An item is
+// `stages` stages of 64 inputs, each as long as its MMAs (2 clocks per activation row by pairs; 2.6, above 128 rows 2.8, in the one-CTA form, which reads all of the
+// activations through its own shared memory) but never less than the decode of its weights, and an epilogue of 760 clocks per 32 rows. Items of up to 128 rows
+// alternate two accumulators: the epilogue of one runs under the next. Wider ones use both, their epilogue is exposed. Launching pairs costs 2900 clocks more.
+// Fitted to 1900 timings (four formats, 2048 to 16384 outputs, 256 to 27648 inputs, 64 to 4001 rows, every form): the form it picks is on average 0.2 %, at most 5 %
+// slower than the best one. Q4_K 8192 x 1024, 2048 rows: pairs of 256 rows 37.6 us, one CTA of 128 rows 32.9; 300 rows of 2048 x 512 9.2 / 6.8; 96 rows of
+// 13824 x 5120 23.7 / 22.7. Items below 64 rows only where m has no more.
+// The candidates are the item sizes, not the numbers of items, so any m has the same few of them.
+// clocks that the decoders take for 64 inputs of 128 outputs (one CTA, 128 rows of 8192 x 4096, less the start and the epilogue)
+constexpr double KQ_DEC_CLOCKS[KYB_FMT_COUNT] = {330.0, 400.0, 356.0, 381.0, 394.0, 345.0, 418.0, 555.0};
 struct KqForm {
     bool pair;
     int mt;
+    double clocks;
 };
-KqForm kq_choose(int64_t n, int64_t m, int nb, int ksplit, int sms, int pairs) {
-    const double stages = 4.0 * nb / ksplit;
-    double c1 = 0.0, c2 = 0.0;
-    const int mt1 = kq_rows_per_item(m, (n + 127) / 128 * ksplit, sms, stages, 300.0, &c1);
-    const int mt2 = pairs > 0 ? kq_rows_per_item(m, (n + 255) / 256 * ksplit, pairs, stages, 300.0, &c2) : 0;
-    if (pairs > 0 && c2 <= 1.02 * c1) return {true, mt2};
-    return {false, mt1};
+KqForm kq_choose(int fmt, int64_t n, int64_t m, int nb, int ksplit, int sms, int pairs) {
+    const double stages = 4.0 * nb / ksplit, dec = KQ_DEC_CLOCKS[fmt];
+    KqForm best{false, 0, 0.0};
+    for (int pair = pairs > 0 ? 1 : 0; pair >= 0; --pair) {
+        const int64_t tiles_n = (pair ? (n + 255) / 256 : (n + 127) / 128) * ksplit, units = pair ? pairs : sms;
+        bool any = false;
+        for (int mt = 256; mt >= 32; mt -= 32) {
+            const int64_t tm = (m + mt - 1) / mt;
+            if ((m + tm * 32 - 1) / (tm * 32) * 32 != mt) continue;                    // as many items of fewer rows cover m: that size is the candidate
+            if (mt < 64 && any) break;
+            any = true;
+            const int64_t rounds = (tiles_n * tm + units - 1) / units;
+            const double walk = stages * std::max(pair ? 1.02 * dec : dec, (pair ? 2.0 : mt > 128 ? 2.8 : 2.59) * mt), epi = 760.0 * (mt / 32);
+            const double clocks = (pair ? 10850.0 : 7920.0) + (mt > 128 ? (double)rounds * (walk + epi + 160.0) : (double)rounds * std::max(walk + 1417.0, epi + 144.0) + epi);
+            if (!best.mt || clocks < best.clocks) best = {pair != 0, mt, clocks};
+        }
+    }
+    return best;
+}
+
+// CTA pairs the device holds at once; without a device half of the SMs
+int kq_pairs(int fmt) {
+    int pairs = 0, dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || kq_configure<true>(fmt, &pairs) != KYB_OK) pairs = kq_sms() / 2;
+    (void)cudaGetLastError();
+    return pairs;
 }
 
 }  // namespace
@@ -1127,7 +1166,7 @@ static int kq_dense(int fmt, const void* t16, int64_t n, int64_t k, const void* 
     const int sms = kq_sms();
     if (msub == 0)
         if (int rc = kq_configure<true>(fmt, &pairs)) return rc;
-    const KqForm form = msub ? KqForm{false, 128 * msub} : kq_choose(n, m, p.nb, ksplit, sms, pairs);
+    const KqForm form = msub ? KqForm{false, 128 * msub, 0.0} : kq_choose(fmt, n, m, p.nb, ksplit, sms, pairs);
     const bool pair = form.pair;
     p.mt = form.mt;
     CUtensorMap ta;                                                                 // one box is 64 inputs of all the rows that a CTA loads for an item
@@ -1167,10 +1206,7 @@ extern "C" int kyb_gemm_kq(int fmt, const void* t16, int64_t n, int64_t k, const
 // Without a device: as on 148 SMs.
 extern "C" int kyb_gemm_kq_plan(int fmt, int64_t n, int64_t k, int64_t m, int split, int64_t* out3) {
     KYB_REQUIRE(fmt >= 0 && fmt < KYB_FMT_COUNT && n > 0 && m > 0 && k > 0 && k % 256 == 0 && split >= 1 && split <= 8 && out3, "bad arguments");
-    int pairs = 0, dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || kq_configure<true>(fmt, &pairs) != KYB_OK) pairs = kq_sms() / 2;
-    (void)cudaGetLastError();
-    const KqForm f = kq_choose(n, m, (int)(k / 256), split, kq_sms(), pairs);
+    const KqForm f = kq_choose(fmt, n, m, (int)(k / 256), split, kq_sms(), kq_pairs(fmt));
     out3[0] = f.pair, out3[1] = f.mt, out3[2] = (f.pair ? (n + 255) / 256 : (n + 127) / 128) * ((m + f.mt - 1) / f.mt) * split;
     return KYB_OK;
 }
