@@ -1114,7 +1114,7 @@ struct KqForm {
     int mt;
     double clocks;
 };
-KqForm kq_choose(int fmt, int64_t n, int64_t m, int nb, int ksplit, int sms, int pairs) {
+KqForm kq_choose(int fmt, int64_t n, int64_t m, int nb, int ksplit, int sms, int pairs, double epi32 = 760.0) {
     const double stages = 4.0 * nb / ksplit, dec = KQ_DEC_CLOCKS[fmt];
     KqForm best{false, 0, 0.0};
     for (int pair = pairs > 0 ? 1 : 0; pair >= 0; --pair) {
@@ -1126,7 +1126,7 @@ KqForm kq_choose(int fmt, int64_t n, int64_t m, int nb, int ksplit, int sms, int
             if (mt < 64 && any) break;
             any = true;
             const int64_t rounds = (tiles_n * tm + units - 1) / units;
-            const double walk = stages * std::max(pair ? 1.02 * dec : dec, (pair ? 2.0 : mt > 128 ? 2.8 : 2.59) * mt), epi = 760.0 * (mt / 32);
+            const double walk = stages * std::max(pair ? 1.02 * dec : dec, (pair ? 2.0 : mt > 128 ? 2.8 : 2.59) * mt), epi = epi32 * (mt / 32);
             const double clocks = (pair ? 10850.0 : 7920.0) + (mt > 128 ? (double)rounds * (walk + epi + 160.0) : (double)rounds * std::max(walk + 1417.0, epi + 144.0) + epi);
             if (!best.mt || clocks < best.clocks) best = {pair != 0, mt, clocks};
         }
@@ -1211,32 +1211,25 @@ extern "C" int kyb_gemm_kq_plan(int fmt, int64_t n, int64_t k, int64_t m, int sp
     return KYB_OK;
 }
 
-// Split-k for products with fewer output tiles than SMs (e.g. 2048 x 3072 outputs from 12288 inputs: 96 tiles of 256 x 256): the k-blocks are cut into `split`
-// equal ranges, (tile, range) items fill the SMs, every item leaves its fp32 accumulator in the workspace and a second kernel adds the ranges in k order (the result
-// is deterministic; it differs from the unsplit product by fp32 summation order only). kyb_gemm_kq_split: the factor the library suggests (1: do not split);
+// Split-k for products that leave most SMs idle (e.g. 300 x 768 outputs from 12288 inputs: 3 items of 256 outputs): the k-blocks are cut into `split` equal ranges,
+// (tile, range) items fill the SMs, every item leaves its fp32 accumulator in the workspace and a second kernel adds the ranges in k order (the result is
+// deterministic; it differs from the unsplit product by fp32 summation order only). kyb_gemm_kq_split: the factor the library suggests (1: do not split);
 // kyb_gemm_kq_split_bytes: bytes of 16-byte aligned workspace the call then needs.
 extern "C" int kyb_gemm_kq_split(int fmt, int64_t n, int64_t k, int64_t m) {
     if (fmt < 0 || fmt >= KYB_FMT_COUNT || n <= 0 || k <= 0 || k % 256 || m <= 128) return 1;
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) (void)cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    (void)cudaGetLastError();
-    const int64_t tiles = ((n + 255) / 256) * ((m + 255) / 256), nb = k / 256;
-    if (tiles >= sms) return 1;                                                       // whole rounds of tiles already fill the SMs
-    // Cost model in microseconds, fitted to measurements with 2048 rows on 3072 x 12288, 1536 x 12288 and 768 x 12288: a 64-input stage of a two-block item of
-    // the one-CTA kernel takes 0.73 us, a 128-input stage of the pair kernel 0.87 us, an item 6 us more (start, exposed epilogue); the split form pays about 10 us
-    // for its second launch and moves (ranges + 0.5) x the fp32 output at about 3 MB per us. The unsplit product is whichever kernel the launcher would take
-    // (pairs unless the tile count lies between the pair count and the SM count). A split must be at least 15 % faster than that.
-    const double out_mb = (double)(((m + 255) / 256) * 256) * (double)(((n + 255) / 256) * 256) * 4.0 / 1.0e6;
-    const int64_t pairs = sms / 2;
-    double whole = 4.0 * nb * 0.73 + 6.0;                                              // fewer tiles than SMs: one round
-    if (!(tiles > pairs && tiles <= 2 * pairs)) whole = std::min(whole, (double)((tiles + pairs - 1) / pairs) * (2.0 * nb * 0.87 + 6.0));
+    const int nb = (int)(k / 256), pairs = kq_pairs(fmt);
+    if ((double)n * (double)m > 32.0 * 1024 * 1024) return 1;                          // hundreds of items: the ranges only add traffic
+    // The launcher's own cost model with the split form's epilogue (fp32 stores, 1300 clocks per 32 rows), 3.2 us for the second launch, and the ranges and the output
+    // at 1.5 and 3.7 MB per us; a split must be 4 % faster. Fitted to 480 timings of 11 shapes, 64 to 2048 rows, Q4_K and Q6_K: from 129 rows on it is on average 0.3 %
+    // slower than the best factor and never slower than no split. Q4_K 768 x 12288, 300 rows 37.9 -> 19.3 us (six ranges), 2048 rows stay at 40.3 (six ranges: 60.9); 2048 x 8192, 512 rows
+    // 28.1 (four ranges: 33.5); 3072 x 12288, 300 rows 38.9 -> 31.3 (three; six: 40.6).
+    const double whole = kq_choose(fmt, n, m, nb, 1, kq_sms(), pairs).clocks / 1900.0;
     int best = 1;
-    double best_cost = 0.85 * whole;
+    double best_us = 0.96 * whole;
     for (int sp = 2; sp <= 8; ++sp) {
-        if (nb % sp || nb / sp < 8) continue;                                           // equal ranges of at least 2048 inputs
-        const double rounds = (double)((tiles * sp + sms - 1) / sms);
-        const double cost = rounds * (4.0 * (double)(nb / sp) * 0.73 + 6.0) + 10.0 + (sp + 0.5) * out_mb / 3.0;
-        if (cost < best_cost) best = sp, best_cost = cost;
+        if (nb % sp || nb / sp < 4) continue;                                           // equal ranges of at least 1024 inputs
+        const double us = kq_choose(fmt, n, m, nb, sp, kq_sms(), pairs, 1300.0).clocks / 1900.0 + 3.2 + (double)m * (double)n / 1.0e6 * (sp * 4 * 0.654 + 2 * 0.273);
+        if (us < best_us) best = sp, best_us = us;
     }
     return best;
 }

@@ -111,7 +111,8 @@ def test_split_k_adds_the_ranges_in_k_order(fmt):
         assert torch.allclose(ys.float(), y1.float(), rtol=2e-3, atol=2e-3 * want.abs().max().item())
     ops.check_device_status()
     L = _lib.lib()
-    assert L.kyb_gemm_kq_split(ops._fmt("q3_k"), 768, 12288, 2048) == 6                       # 24 tiles of 256 x 256 on 148 SMs: sixths fill one round
+    split = lambda n, k, m: L.kyb_gemm_kq_split(ops._fmt("q3_k"), n, k, m)
+    assert split(768, 12288, 300) == 6 and split(768, 12288, 2048) == 1                     # 9 items leave most SMs idle; 72 of 256 rows don't (six ranges: 1.5 times the time)
     assert L.kyb_gemm_kq_split(ops._fmt("q3_k"), 12288, 3072, 2048) == 1 and L.kyb_gemm_kq_split(ops._fmt(fmt), n, 2048, m) == 1
     y = torch.empty((m, n), dtype=torch.float16, device="cuda")
     small = torch.empty(1 << 20, dtype=torch.uint8, device="cuda")
