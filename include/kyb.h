@@ -129,8 +129,8 @@ int kyb_gemm_nvfp4_ag(const void* a_codes, const void* sfa, const void* b_codes,
  * form with up to that many 128-row blocks of a per work item (same bits either way). The grouped form needs n % 256 == 0 and tb / off from
  * kyb_moe_plan with the same mt (128 or 256 rows of one expert per work item). */
 int kyb_gemm_kq(int fmt, const void* t16, int64_t n, int64_t k, const void* a, int64_t lda, int64_t m, float gscale, void* d, int64_t ldd, int msub, void* stream);
-/* diagnostics: the form a shape takes with msub = 0. out3 = {1 CTA pairs / 0 one CTA, activation rows per work item, work items}; works without a device */
-int kyb_gemm_kq_plan(int fmt, int64_t n, int64_t k, int64_t m, int split, int64_t* out3);
+/* diagnostics: the form a shape takes with msub = 0 (destinations > 1: kyb_gemm_kq_ag). out3 = {1 CTA pairs / 0 one CTA, activation rows per work item, work items}; works without a device */
+int kyb_gemm_kq_plan(int fmt, int64_t n, int64_t k, int64_t m, int split, int destinations, int64_t* out3);
 /* split-k form of kyb_gemm_kq for products with fewer 256 x 256 output tiles than SMs (the reference has no counterpart: its fallback for these row counts is
  * dequantise + library matmul, kyojin_mlx/foreign_linear.py:710 / :737). The 256-input blocks are cut into `split` equal ranges, (tile, range) items fill the
  * SMs, every item leaves its fp32 accumulator in the workspace, a second kernel adds the ranges in k order, scales, saturates and stores d. Deterministic; differs

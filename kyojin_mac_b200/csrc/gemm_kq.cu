@@ -1114,13 +1114,13 @@ struct KqForm {
     int mt;
     double clocks;
 };
-KqForm kq_choose(int fmt, int64_t n, int64_t m, int nb, int ksplit, int sms, int pairs, double epi32 = 760.0) {
+KqForm kq_choose(int fmt, int64_t n, int64_t m, int nb, int ksplit, int sms, int pairs, int widest = 256, double epi32 = 760.0) {
     const double stages = 4.0 * nb / ksplit, dec = KQ_DEC_CLOCKS[fmt];
     KqForm best{false, 0, 0.0};
     for (int pair = pairs > 0 ? 1 : 0; pair >= 0; --pair) {
         const int64_t tiles_n = (pair ? (n + 255) / 256 : (n + 127) / 128) * ksplit, units = pair ? pairs : sms;
         bool any = false;
-        for (int mt = 256; mt >= 32; mt -= 32) {
+        for (int mt = widest; mt >= 32; mt -= 32) {
             const int64_t tm = (m + mt - 1) / mt;
             if ((m + tm * 32 - 1) / (tm * 32) * 32 != mt) continue;                    // as many items of fewer rows cover m: that size is the candidate
             if (mt < 64 && any) break;
@@ -1133,6 +1133,11 @@ KqForm kq_choose(int fmt, int64_t n, int64_t m, int nb, int ksplit, int sms, int
     }
     return best;
 }
+
+// Several destinations: an item's stores to the other GPUs take longer than its MMAs (256 x 256 outputs to seven peers are 0.9 MB, 88 us of a pair's share of the link
+// against 30 us of MMAs at 7168 inputs), so the items stay at 128 rows, whose epilogue runs under the next item's MMAs. Reasoned, not measured on several GPUs; with all
+// destinations on one GPU the narrow items cost 0 to 10 %.
+int kq_widest(int nout) { return nout > 1 ? 128 : 256; }
 
 // CTA pairs the device holds at once; without a device half of the SMs
 int kq_pairs(int fmt) {
@@ -1166,7 +1171,7 @@ static int kq_dense(int fmt, const void* t16, int64_t n, int64_t k, const void* 
     const int sms = kq_sms();
     if (msub == 0)
         if (int rc = kq_configure<true>(fmt, &pairs)) return rc;
-    const KqForm form = msub ? KqForm{false, 128 * msub, 0.0} : kq_choose(fmt, n, m, p.nb, ksplit, sms, pairs);
+    const KqForm form = msub ? KqForm{false, 128 * msub, 0.0} : kq_choose(fmt, n, m, p.nb, ksplit, sms, pairs, kq_widest(nout));
     const bool pair = form.pair;
     p.mt = form.mt;
     CUtensorMap ta;                                                                 // one box is 64 inputs of all the rows that a CTA loads for an item
@@ -1202,11 +1207,11 @@ extern "C" int kyb_gemm_kq(int fmt, const void* t16, int64_t n, int64_t k, const
     return kq_dense(fmt, t16, n, k, a, lda, m, gscale, outs, 1, ldd, 0, msub, stream);
 }
 
-// Diagnostics: the form that kyb_gemm_kq (split = 1) or kyb_gemm_kq_splitk takes for a shape. out3 = {1 by CTA pairs / 0 one CTA, activation rows per item, items}.
+// Diagnostics: the form that kyb_gemm_kq (split = 1), kyb_gemm_kq_splitk or kyb_gemm_kq_ag (destinations > 1) takes for a shape. out3 = {1 by CTA pairs / 0 one CTA, activation rows per item, items}.
 // Without a device: as on 148 SMs.
-extern "C" int kyb_gemm_kq_plan(int fmt, int64_t n, int64_t k, int64_t m, int split, int64_t* out3) {
-    KYB_REQUIRE(fmt >= 0 && fmt < KYB_FMT_COUNT && n > 0 && m > 0 && k > 0 && k % 256 == 0 && split >= 1 && split <= 8 && out3, "bad arguments");
-    const KqForm f = kq_choose(fmt, n, m, (int)(k / 256), split, kq_sms(), kq_pairs(fmt));
+extern "C" int kyb_gemm_kq_plan(int fmt, int64_t n, int64_t k, int64_t m, int split, int destinations, int64_t* out3) {
+    KYB_REQUIRE(fmt >= 0 && fmt < KYB_FMT_COUNT && n > 0 && m > 0 && k > 0 && k % 256 == 0 && split >= 1 && split <= 8 && destinations >= 1 && out3, "bad arguments");
+    const KqForm f = kq_choose(fmt, n, m, (int)(k / 256), split, kq_sms(), kq_pairs(fmt), kq_widest(destinations));
     out3[0] = f.pair, out3[1] = f.mt, out3[2] = (f.pair ? (n + 255) / 256 : (n + 127) / 128) * ((m + f.mt - 1) / f.mt) * split;
     return KYB_OK;
 }
@@ -1228,7 +1233,7 @@ extern "C" int kyb_gemm_kq_split(int fmt, int64_t n, int64_t k, int64_t m) {
     double best_us = 0.96 * whole;
     for (int sp = 2; sp <= 8; ++sp) {
         if (nb % sp || nb / sp < 4) continue;                                           // equal ranges of at least 1024 inputs
-        const double us = kq_choose(fmt, n, m, nb, sp, kq_sms(), pairs, 1300.0).clocks / 1900.0 + 3.2 + (double)m * (double)n / 1.0e6 * (sp * 4 * 0.654 + 2 * 0.273);
+        const double us = kq_choose(fmt, n, m, nb, sp, kq_sms(), pairs, 256, 1300.0).clocks / 1900.0 + 3.2 + (double)m * (double)n / 1.0e6 * (sp * 4 * 0.654 + 2 * 0.273);
         if (us < best_us) best = sp, best_us = us;
     }
     return best;

@@ -382,11 +382,11 @@ def gemm_kq(fmt, t16: torch.Tensor, n: int, k: int, a: torch.Tensor, gscale: flo
     return d
 
 
-def gemm_kq_plan(fmt, n: int, k: int, m: int, split: int = 1) -> dict:
-    """The form gemm_kq takes for a shape: by CTA pairs or not, activation rows per work item, work items."""
+def gemm_kq_plan(fmt, n: int, k: int, m: int, split: int = 1, destinations: int = 1) -> dict:
+    """The form gemm_kq (several destinations: gemm_kq_ag) takes for a shape: by CTA pairs or not, activation rows per work item, work items."""
     import ctypes
     out = (ctypes.c_int64 * 3)()
-    _lib.check(_lib.lib().kyb_gemm_kq_plan(_fmt(fmt), n, k, m, split, out))
+    _lib.check(_lib.lib().kyb_gemm_kq_plan(_fmt(fmt), n, k, m, split, destinations, out))
     return dict(pair=bool(out[0]), rows=out[1], items=out[2])
 
 

@@ -27,6 +27,14 @@ def test_plans_are_runnable(fmt, split):
             assert p["items"] == tiles * ((m + p["rows"] - 1) // p["rows"]) * split, where
 
 
+@pytest.mark.parametrize("n,k,m", [(8192, 7168, 2048), (2048, 7168, 2048), (1536, 3072, 4096), (7168, 18432, 1024)])
+def test_items_of_several_destinations_stay_narrow(n, k, m):
+    """Up to 128 rows an item's epilogue (stores to all ranks) runs under the next item's MMAs; wider items would make the MMAs wait for the stores."""
+    assert ops.gemm_kq_plan("q4_k", n, k, m)["rows"] > 128
+    for destinations in (2, 4, 8):
+        assert ops.gemm_kq_plan("q4_k", n, k, m, destinations=destinations)["rows"] <= 128
+
+
 @pytest.mark.gpu
 def test_more_than_a_million_rows():
     """2^20 + 33 rows (4097 items of 256 rows): the result is that of the same rows in a small product, bit for bit."""
