@@ -29,7 +29,7 @@ extern "C" {
 #define KYB_EINVAL       -1   /* bad shape, alignment, format or null pointer */
 #define KYB_ECUDA        -2   /* a CUDA runtime call failed (message in kyb_last_error) */
 #define KYB_ETIMEOUT     -3   /* a bounded device-side wait expired (reported through the status word) */
-#define KYB_EUNSUPPORTED -4   /* valid request outside what this build implements */
+#define KYB_EUNSUPPORTED -4   /* valid request outside what this build implements (no entry returns it at present) */
 #define KYB_EWORKSPACE   -5   /* scratch buffer missing or too small */
 
 /* weight formats (GGUF block types of kyojin_mlx/foreign_gguf.py:27-35 TYPES; NVFP4 also in the qs/meta pack form) */
@@ -252,6 +252,8 @@ int kyb_gemv_t16_static(int fmt, const void* t16, int64_t n, int64_t k, const vo
  * chunk sums through the workspace and a finalize launch; 2: whole row tiles per CTA, chunk sums added in shared memory, one launch), warps per CTA, k-blocks
  * per canonical chunk, k-blocks per part, k parts, dynamic shared memory bytes, CTAs}. */
 int kyb_gemv_plan(int fmt, int64_t n, int64_t k, int64_t m, int* out8);
+/* the same for a caller that brings workspace_bytes of scratch (kyb_gemv_t16: another form where the best one needs more; 0 warps: none fits) */
+int kyb_gemv_plan_within(int fmt, int64_t n, int64_t k, int64_t m, size_t workspace_bytes, int* out8);
 
 /* device status word of the calling thread's current device: nonzero after a bounded wait expired inside a kernel.
  * kyb_check_device_status synchronises `stream`, reads and clears it. */

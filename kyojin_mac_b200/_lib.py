@@ -159,6 +159,7 @@ SIGNATURES = {
     "kyb_moe_groups": (_int, [_vp, _i64, _int, _vp, _vp, _vp, _vp]),
     "kyb_gemv_group_t16": (_int, [_int, _vp, _vp, _i64, _i64, _int, _vp, _vp, _f32, _i64, _vp, _vp, _int, _i64, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp]),
     "kyb_gemv_plan": (_int, [_int, _i64, _i64, _i64, C.POINTER(C.c_int)]),
+    "kyb_gemv_plan_within": (_int, [_int, _i64, _i64, _i64, _sz, C.POINTER(C.c_int)]),
     "kyb_check_device_status": (_int, [_vp]),
     "kyb_selftest_wait_timeout": (_int, [_int, _vp]),
 }

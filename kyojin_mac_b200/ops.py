@@ -134,10 +134,12 @@ def gemm_f16(a: torch.Tensor, b: torch.Tensor, gscale: float = 1.0, out: torch.T
     return d
 
 
-def gemv_plan(fmt, n: int, k: int, m: int) -> dict:
+def gemv_plan(fmt, n: int, k: int, m: int, workspace_bytes: int | None = None) -> dict:
+    """How a decode product is launched; workspace_bytes: for a caller that brings that much scratch (None: as much as the best form wants)."""
     import ctypes
     out = (ctypes.c_int * 8)()
-    _lib.check(_lib.lib().kyb_gemv_plan(_fmt(fmt), n, k, m, out))
+    L = _lib.lib()
+    _lib.check(L.kyb_gemv_plan(_fmt(fmt), n, k, m, out) if workspace_bytes is None else L.kyb_gemv_plan_within(_fmt(fmt), n, k, m, workspace_bytes, out))
     return dict(zip(("nt", "aligned", "warps", "kc", "kbp", "ksplit", "smem", "grid"), list(out)))
 
 

@@ -6,9 +6,10 @@ import pytest
 import torch
 
 from kyojin_mac_b200 import ops, synth
-from kyojin_mac_b200.layout import FMT_ID
+from kyojin_mac_b200.layout import FMT_ID, TILE_BYTES
 
 KC_MAX, SMEM_MAX, SMS = 8, 226 * 1024, 148
+MINS = {"q4_k": 256, "q5_k": 256, "q2_k": 512}          # staged sums per block and column tile
 
 
 @pytest.mark.parametrize("fmt", sorted(FMT_ID))
@@ -23,6 +24,26 @@ def test_plans_are_runnable(fmt):
         assert p["kbp"] * p["ksplit"] >= nb and p["kbp"] * (p["ksplit"] - 1) < nb and p["grid"] % p["ksplit"] == 0, where   # the parts cover k and none is empty
         assert p["kbp"] == nb or p["kbp"] % p["kc"] == 0, where                              # a part is whole chunks
         assert (ops.gemv_workspace_bytes(fmt, n, nb * 256, m) > 0) == (p["aligned"] == 0 or (p["aligned"] == 1 and p["ksplit"] > 1)), where
+
+
+@pytest.mark.parametrize("fmt", sorted(FMT_ID))
+def test_plans_without_a_workspace_are_runnable(fmt):
+    """A caller without scratch gets a form without chunk sums in memory that the kernel can run, wherever such a form fits shared memory; nothing fits only where
+    the staged activations of all of k do not."""
+    rng = random.Random(100 + FMT_ID[fmt])
+    served = 0
+    for _ in range(300):
+        n, nb, m = int(2 ** rng.uniform(0, 17)), int(2 ** rng.uniform(0, 8)), rng.randint(1, 32)
+        p = ops.gemv_plan(fmt, n, nb * 256, m, 0)
+        where = (fmt, n, nb * 256, m, p)
+        two_launches = p["aligned"] == 0 or (p["aligned"] == 1 and p["ksplit"] > 1)
+        if two_launches:                                                                     # refused by the product for want of a workspace
+            staged = nb * (16 * p["nt"] * min(8, 1 << max(0, (m - 1).bit_length())) * 32 + MINS.get(fmt, 0) * p["nt"])
+            assert staged + 4 * (2 * TILE_BYTES[fmt] + 1312) > SMEM_MAX, where               # rings, scale scratch and barriers of four warps
+            continue
+        served += 1
+        assert p["ksplit"] == 1 and p["kbp"] == nb and p["smem"] <= SMEM_MAX and 4 <= p["warps"] <= 12 and p["grid"] <= SMS, where
+    assert served >= 100
 
 
 @pytest.mark.gpu
@@ -49,8 +70,7 @@ def test_rows_do_not_depend_on_the_plan(fmt, n, k):
 def test_products_without_a_workspace(fmt, n, k, m):
     """A shape whose best plan uses a workspace although another form serves it: a caller without one gets that form, the same bits."""
     from kyojin_mac_b200 import _lib
-    if ops.gemv_workspace_bytes(fmt, n, k, m) == 0:
-        pytest.skip("the best plan needs no workspace here")
+    assert ops.gemv_workspace_bytes(fmt, n, k, m) > 0 and ops.gemv_plan(fmt, n, k, m, 0)["aligned"] == 1
     t16 = synth.t16_random_device(fmt, n, k, seed=7)
     x = torch.randn((m, k), device="cuda").to(torch.float16)
     y = torch.empty((m, n), dtype=torch.float16, device="cuda")
