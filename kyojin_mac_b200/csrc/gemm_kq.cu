@@ -9,7 +9,7 @@
 // 128-row blocks, and the accumulator holds D transposed (lanes = outputs, columns = activation rows).
 //
 // One persistent CTA per SM, 22 warps:
-//   warp 0      TMA: activation boxes (64 rows x 64 inputs) into a ring of shared-memory stages
+//   warp 0      TMA: activation boxes (64 inputs of all the rows that the CTA needs for an item; grouped form: of 64 rows) into a ring of shared-memory stages
 //   warp 1      tcgen05.mma issuer (M = 128 output rows, A from tensor memory, two accumulator slots of 128 columns), tcgen05.commit hands stages back
 //   warps 2-5   epilogue: tcgen05.ld 16x256b, output scale, stmatrix.trans turns the fragments around into [activation row][output] staging tiles, which leave as
 //               tiled bulk stores (two warps per store of 32 rows x 64 outputs) or as coalesced row pieces
@@ -17,7 +17,7 @@
 //               quarter q) and every second T16 tile of it (parity j >> 1). It keeps one T16 tile in registers, each unit refilled from its next tile right after its
 //               use (across items too), unpacks a 64-input quarter with LOP3 / PRMT into fp16 pairs, applies the block scales with half2 arithmetic (scale and
 //               min rounded to fp16, then one fma per pair: the rounding points of the reference's few-row kernels, kyojin_mlx/foreign_metal.py:1357-1358,
-//               :1382-1383) and stores it into one of eight tensor-memory stages (32 columns each).
+//               :1382-1383) and stores it into half of one of four tensor-memory stages (64 columns each).
 // PAIR (tcgen05 cta_group::2): two CTAs of neighbouring SMs compute 256 outputs; each decodes its own 128 rows into its own tensor memory and loads half of the
 // activation rows, one MMA of the leader (cluster rank 0) drives both tensor cores. full barriers, acc_empty in the leader; empty and acc_full in each CTA
 // (commit to the pair). Remote arrivals use the plain (CTA-scope release) form: what they publish sits in the arriving CTA's own tensor memory.
@@ -231,8 +231,6 @@ __device__ __forceinline__ void kq_load(const uint8_t* tile, int lane, KqTile<FM
     }
 }
 
-// Block scales of the tile as half2 pairs (value, value) in the warp's scratch. Q4_K: S[row][8] at row * 32, Z[row][8] at 512 + row * 32 (scale and minus min of
-// the eight 32-input sub-blocks); the others: S[row][16] at row * 80 (one scale per 16 inputs; the 80-byte pitch keeps the 16-byte reads of 8 rows on distinct banks).
 // (lo, hi) fp16 pair -> the two (v, v) pairs, clamped to the finite fp16 range (an overflowing block scale must not turn into inf * 0)
 __device__ __forceinline__ uint32_t h2_clamp(uint32_t a) {
     __half2 v = *reinterpret_cast<__half2*>(&a);
@@ -268,13 +266,13 @@ __device__ __forceinline__ void kq_prep_scales(const KqTile<FMT>& tr, uint32_t s
             sts128(scr + r * 80 + 32 * hf + 16 * q, make_uint4(prmt(sa, za, 0x5410u), prmt(sa, za, 0x7632u), prmt(sb, zb, 0x5410u), prmt(sb, zb, 0x7632u)));
         }
     } else if constexpr (FMT == KYB_FMT_IQ4_XS) {
-        // 6-bit scales of sub-blocks 4 hf .. 4 hf + 3 (4 low bits from scales_l, 2 high bits from scales_h), minus 32, times d: S[row][8] as (v, v) pairs at row * 32
+        // 6-bit scales of sub-blocks 4 hf .. 4 hf + 3 (4 low bits from scales_l, 2 high bits from scales_h), minus 32, times d: S[row][8] as (v, v) pairs at row * 48
         const uint32_t sh = tr.sc.x >> (16 + 8 * hf), sl = tr.sc.y >> (16 * hf);
         const uint32_t lsw = ((sl & 15u) | ((sh & 3u) << 4)) | ((((sl >> 4) & 15u) | (((sh >> 2) & 3u) << 4)) << 8) | ((((sl >> 8) & 15u) | (((sh >> 4) & 3u) << 4)) << 16) |
                              ((((sl >> 12) & 15u) | (((sh >> 6) & 3u) << 4)) << 24);
         sts128(scr + r * 48 + 16 * hf, kq_scale4(lsw, 0x64206420u, prmt(tr.sc.x, 0u, 0x1010u)));
     } else if constexpr (FMT == KYB_FMT_Q8_0) {
-        // one fp16 d per 32 inputs: S[row][8] as (d, d) pairs at row * 32 (lane half hf covers blocks 4 hf .. 4 hf + 3)
+        // one fp16 d per 32 inputs: S[row][8] as (d, d) pairs at row * 48 (lane half hf covers blocks 4 hf .. 4 hf + 3)
         const uint32_t w0 = hf ? tr.sc.z : tr.sc.x, w1 = hf ? tr.sc.w : tr.sc.y;
         sts128(scr + r * 48 + 16 * hf, make_uint4(h2_clamp(prmt(w0, 0u, 0x1010u)), h2_clamp(prmt(w0, 0u, 0x3232u)), h2_clamp(prmt(w1, 0u, 0x1010u)), h2_clamp(prmt(w1, 0u, 0x3232u))));
     } else if constexpr (FMT == KYB_FMT_Q4_K || FMT == KYB_FMT_Q5_K) {

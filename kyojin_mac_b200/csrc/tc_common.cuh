@@ -45,7 +45,8 @@ static inline int kyb_make_tmap_2d(CUtensorMap* tm, CUtensorMapDataType dt, int 
     return KYB_OK;
 }
 
-// Tensor maps of the output matrix on every receiving rank (one entry without sharding): 16-bit elements, box 32 rows x 32 columns, 64-byte swizzle.
+// Tensor maps of the output matrix on every receiving rank (one entry without sharding): 16-bit elements, boxes of 32 rows x 32 columns with 64-byte swizzle
+// (epilogue_stage_store) or 32 x 64 with 128-byte swizzle (epilogue_stage_store_wide and the K-quant GEMM).
 struct KybOutMaps {
     CUtensorMap m[8];
 };
@@ -196,13 +197,6 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
 
 // arrival on a barrier of the other CTA of the pair (bar: shared::cluster address), default semantics (release at CTA scope)
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 
 __device__ __forceinline__ bool elect_one() {
     uint32_t pred;
