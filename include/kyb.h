@@ -125,17 +125,17 @@ int kyb_gemm_nvfp4_ag(const void* a_codes, const void* sfa, const void* b_codes,
  * matrix never exists in HBM. d fp16 [m, n] = sat(gscale * a fp16 [m, k] x W^T). Same call sites as the two entries above
  * (kyojin_mlx/foreign_linear.py:710 / :737 dense, kyojin_mlx/foreign_kqgmm.py:225-239 `gmm` grouped). Weights are rounded to fp16 at the reference's own rounding
  * points for its few-row tensor kernels (block scale and min to fp16, one fp16 fma per weight: kyojin_mlx/foreign_metal.py:1357-1358, :1382-1383); NVFP4 weights
- * are exact in fp16. msub = 0: chosen by the library (CTA pairs, tcgen05 cta_group::2, unless the one-CTA form fills the SMs better); 1 or 2: the one-CTA
+ * are exact in fp16. msub = 0: chosen by the library (CTA pairs, tcgen05 cta_group::2, unless the one-CTA form is the faster one); 1 or 2: the one-CTA
  * form with up to that many 128-row blocks of a per work item (same bits either way). The grouped form needs n % 256 == 0 and tb / off from
  * kyb_moe_plan with the same mt (128 or 256 rows of one expert per work item). */
 int kyb_gemm_kq(int fmt, const void* t16, int64_t n, int64_t k, const void* a, int64_t lda, int64_t m, float gscale, void* d, int64_t ldd, int msub, void* stream);
 /* diagnostics: the form a shape takes with msub = 0 (destinations > 1: kyb_gemm_kq_ag). out3 = {1 CTA pairs / 0 one CTA, activation rows per work item, work items}; works without a device */
 int kyb_gemm_kq_plan(int fmt, int64_t n, int64_t k, int64_t m, int split, int destinations, int64_t* out3);
-/* split-k form of kyb_gemm_kq for products with fewer 256 x 256 output tiles than SMs (the reference has no counterpart: its fallback for these row counts is
+/* split-k form of kyb_gemm_kq for products that leave most SMs idle (the reference has no counterpart: its fallback for these row counts is
  * dequantise + library matmul, kyojin_mlx/foreign_linear.py:710 / :737). The 256-input blocks are cut into `split` equal ranges, (tile, range) items fill the
  * SMs, every item leaves its fp32 accumulator in the workspace, a second kernel adds the ranges in k order, scales, saturates and stores d. Deterministic; differs
  * from kyb_gemm_kq by the fp32 summation order only. kyb_gemm_kq_split: the factor the library suggests for a shape (1: do not split; splits keep ranges of at
- * least 2048 inputs). kyb_gemm_kq_split_bytes: size of the 16-byte aligned workspace = split * (m rounded up to 256) * (n rounded up to 256) * 4. */
+ * least 1024 inputs). kyb_gemm_kq_split_bytes: size of the 16-byte aligned workspace = split * (m rounded up to 256) * (n rounded up to 256) * 4. */
 int kyb_gemm_kq_split(int fmt, int64_t n, int64_t k, int64_t m);
 size_t kyb_gemm_kq_split_bytes(int64_t n, int64_t m, int split);
 int kyb_gemm_kq_splitk(int fmt, const void* t16, int64_t n, int64_t k, const void* a, int64_t lda, int64_t m, float gscale, void* d, int64_t ldd, int split,

@@ -23,11 +23,11 @@
 // (commit to the pair). Remote arrivals use the plain (CTA-scope release) form: what they publish sits in the arriving CTA's own tensor memory.
 // Every mbarrier wait is bounded; a wait that gives up sets the device status word and the CTA drains.
 //
-// What bounds it: wide items (N = 256) the tensor core and, in a long run of them, the power limit; narrow ones the chain of the decoders and of the two issuing warps
-// (about 350 clocks per 64 inputs of 128 outputs). Measured against the form with the decoded weights in shared memory (same box, back-to-back launches):
-// Q4_K 13824 x 5120, 96 rows 50.6 -> 24.8 us; 18944 x 7168, 32 / 128 rows 84 / 85 -> 37 / 43 us; Q6_K 5120 x 27648, 300 rows 146 -> 114 us; Q3_K 3072 x 12288,
-// 2048 rows 169 -> 141 us; Q4_K 16384 x 7168, 4001 rows 826 -> 782 us (power-limited; 664 us in a short burst); 256 experts of 2048 x 7168, 4096 tokens x 8: gate
-// and up 2684 -> 1945 us, down 1450 -> 1264 us. The sums are the same bits: the MMA adds the same products in the same order with its operands exchanged.
+// What bounds it: wide items (N = 256) the tensor core, their exposed epilogue and, in a long run of them, the power limit; narrow ones the decoders (330 clocks per 64
+// inputs of 128 outputs for Q4_K, up to 555 for IQ4_XS, against 256 of MMA at 128 rows); few inputs the epilogue. Measured, the form with the decoded weights in shared
+// memory -> now: Q4_K 13824 x 5120, 96 rows 50.6 -> 24.0 us; 8192 x 4096, 128 rows 40.8 -> 17.5; Q6_K 5120 x 27648, 300 rows 146 -> 114.7; Q3_K 12288 x 3072, 2048
+// rows 156 -> 140, 3072 x 12288 169 -> 138; 256 experts of 2048 x 7168, 4096 tokens x 8, weighted sum included 5055 -> 3996 us. 8192 outputs of 512 or 1024 inputs and
+// 4096 rows are 4 to 12 % slower than in that form. The sums are the same bits: the MMA adds the same products in the same order with its operands exchanged.
 #include <algorithm>
 #include <cstring>
 #include <mutex>

@@ -362,7 +362,7 @@ def gemm_f16_grouped(a: torch.Tensor, b: torch.Tensor, n: int, E: int, tb: torch
 def gemm_kq(fmt, t16: torch.Tensor, n: int, k: int, a: torch.Tensor, gscale: float = 1.0, out: torch.Tensor | None = None, msub: int = 0,
             split: int | None = None) -> torch.Tensor:
     """d fp16 [m, n] = a fp16 [m, k] @ W^T with W decoded from its T16 tiles inside the GEMM (no fp16 copy of W in HBM).
-    split: number of k-ranges (split-k through an fp32 workspace for products with fewer output tiles than SMs); None = the library's suggestion when msub is 0
+    split: number of k-ranges (split-k through an fp32 workspace for products that leave most SMs idle); None = the library's suggestion when msub is 0
     and `flags.GEMM_SPLIT_K` is on, 1 = never."""
     _need_cuda(t16, a)
     if a.dtype != torch.float16 or a.dim() != 2 or a.shape[1] != k:
