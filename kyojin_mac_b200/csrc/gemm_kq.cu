@@ -27,7 +27,7 @@
 // inputs of 128 outputs for Q4_K, up to 555 for IQ4_XS, against 256 of MMA at 128 rows); few inputs the epilogue. Measured, the form with the decoded weights in shared
 // memory -> now: Q4_K 13824 x 5120, 96 rows 50.6 -> 24.0 us; 8192 x 4096, 128 rows 40.8 -> 17.5; Q6_K 5120 x 27648, 300 rows 146 -> 114.7; Q3_K 12288 x 3072, 2048
 // rows 156 -> 140, 3072 x 12288 169 -> 138; 256 experts of 2048 x 7168, 4096 tokens x 8, weighted sum included 5055 -> 3996 us. 8192 outputs of 512 or 1024 inputs and
-// 4096 rows are 4 to 12 % slower than in that form. The sums are the same bits: the MMA adds the same products in the same order with its operands exchanged.
+// 4096 rows are 7 to 14 % slower than in that form. The sums are the same bits: the MMA adds the same products in the same order with its operands exchanged.
 #include <algorithm>
 #include <cstring>
 #include <mutex>
